@@ -113,7 +113,8 @@ struct solar_gpu_context {
         grp_cell, grp_w, w_cnt, w_off, w_tmp, w_cell, w_val, order_first, order_inv, tile_flag, tile_pos,
         tile_start, tile_union, tile_slot, tile_rows, tile_gcnt, tile_gnch, tile_gbase, tile_tbase, tile_table,
         tile_erow, tile_ew, chunk_perm, chunk_flag, chunk_pos, chunk_tmp, mma_union, mma_nch, mma_cbase,
-        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, mma_sched, mma_retry, cone, cone_tmp, cone_specs;
+        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, mma_sched, mma_retry, cone, cone_tmp, cone_specs,
+        sweep_blocks, sweep_line, box;
     int* h_scalars = nullptr;   // pinned host scratch for small read-backs
     long long mem_limit = 0;    // device bytes the buffers may hold (0: no limit)
     size_t dev_total = 0;       // device memory size, read once at creation
@@ -135,6 +136,10 @@ struct solar_gpu_context {
     // solar_gpu_run_batch: the early-exit tables of every tile are built in
     // one buffer (the first context's), tile after tile on one stream
     DevBuf* cone_shared = nullptr;
+    // origin classes of the tracer's tables in sweep_blocks / sweep_line (0:
+    // none built); in a batch, the first context's tables serve every tile
+    int sweep_ne = 0;
+    solar_gpu_context* sweep_owner = nullptr;
     HourLoop hours;
     // per kernel-group event log (time_kernels)
     bool ktime = false;
@@ -144,7 +149,7 @@ struct solar_gpu_context {
     cudaStream_t kt_stream = nullptr;
 };
 
-static constexpr int kNumBufs = 84;
+static constexpr int kNumBufs = 87;
 extern "C" {
 static void all_bufs(solar_gpu_context* c, DevBuf** out);   // defined with the exports below
 }
@@ -444,6 +449,58 @@ int padded_grid(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables&
     return SOLAR_GPU_OK;
 }
 
+// The sweeping tracer's tables, which depend on the directions alone (built
+// when a larger grid than before needs them, and kept in the context), and the
+// box maxima of this call's heights.  New memory for them may take a sixteenth
+// of what is free, and none under a memory limit (a call that fits the limit
+// without them must still fit); without them t.ne is 0 and every ray is walked
+// by itself.
+int sweep_tables(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables& sky, SweepTables& t, cudaStream_t st)
+{
+    solar_gpu_context* own = c->sweep_owner ? c->sweep_owner : c;
+    const int D = (int)sky.dirs.size(), ne = sweep_classes(s->grid_width, s->grid_height);
+    t = SweepTables{};
+    if (ne == 0 || sky.vsize != 18) return SOLAR_GPU_OK;
+    for (int d = 0; d < D; ++d)   // the upper rays of an azimuth share an early-exit table
+        if (d % 36 < 18 && (sky.dirs[d].meta >> 17) != (sky.dirs[d - d % 36].meta >> 17)) return SOLAR_GPU_OK;
+    const size_t cells = (size_t)(s->grid_width + 2) * (size_t)(s->grid_height + 2);
+    const size_t tab = sweep_block_bytes(D, ne), box = 4 * sizeof(float) * cells;
+    const bool build = own->sweep_ne < ne;
+    const size_t grow = (build ? tab : 0) + (own->box.cap < box ? box - own->box.cap : 0);
+    if (grow > 0) {
+        size_t free_b = 0, total_b = 0;
+        if (own->mem_limit > 0 || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || grow > free_b / 16) {
+            (void)cudaGetLastError();
+            return SOLAR_GPU_OK;
+        }
+    }
+    if (build) own->sweep_ne = 0;
+    if ((build && (ensure(own, own->sweep_blocks, tab) != SOLAR_GPU_OK ||
+                   ensure(own, own->sweep_line, sweep_line_bytes(D)) != SOLAR_GPU_OK)) ||
+        ensure(own, own->box, box) != SOLAR_GPU_OK) {
+        (void)cudaGetLastError();   // no room after all
+        return SOLAR_GPU_OK;
+    }
+    t = SweepTables{as<float>(own->sweep_blocks), as<int>(own->sweep_line), build ? ne : own->sweep_ne,
+                    as<float>(own->box), cells};
+    if (build) {
+        CK(launch_sweep_tables(as<DirEntry>(c->dirs), D, t, st));
+        own->sweep_ne = ne;
+        c->launches += 2;
+    }
+    CK(launch_box_max(as<float>(c->gpad), s->grid_width, s->grid_height, as<float>(own->box), cells, st));
+    c->launches += 1;
+    return SOLAR_GPU_OK;
+}
+
+// All directions of chunk_count voxels, by sweeps where there are tables.
+cudaError_t trace_rows(const SweepTables& sweep, const DevScene& ds, const DirEntry* dirs, int D, int words32, int v0,
+                       int n, int* raw, uint32_t* shadow, const int* perm, int* err, cudaStream_t st)
+{
+    return sweep.ne > 0 ? launch_trace_sweep(ds, dirs, D, words32, v0, n, raw, shadow, perm, sweep, err, st)
+                        : launch_trace(ds, dirs, D, words32, v0, n, raw, shadow, perm, err, st);
+}
+
 int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_scene* s,
            const SkyTables& sky, cudaStream_t st, bool want_csr, bool want_barle)
 {
@@ -473,9 +530,11 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
         RK(ensure(c, c->barle_bytes, (size_t)N * 160));
     }
     DevScene ds = dev_scene(s);
+    SweepTables sweep;
     {
         KScope k(c, SOLAR_GPU_KT_TRACE);   // the tracer's inputs count with the tracer
         RK(padded_grid(c, s, sky, ds, st));
+        RK(sweep_tables(c, s, sky, sweep, st));
     }
     // Rows follow the visiting order (Morton-adjacent voxels share a warp, so
     // their rays have similar lengths); with several chunks, each chunk (a
@@ -509,8 +568,8 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
         }
         {
             KScope k(c, SOLAR_GPU_KT_TRACE);
-            CK(launch_trace(ds, as<DirEntry>(c->dirs), D, c->words32, (int)v0, n, as<int>(c->raw),
-                            as<uint32_t>(c->shadow), perm, as<int>(c->err), st));
+            CK(trace_rows(sweep, ds, as<DirEntry>(c->dirs), D, c->words32, (int)v0, n, as<int>(c->raw),
+                          as<uint32_t>(c->shadow), perm, as<int>(c->err), st));
         }
         {
             KScope k(c, SOLAR_GPU_KT_DEDUPE);
@@ -564,7 +623,8 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
     // smaller ones are kept for the next call.
     if (c->raw.cap > c->dev_total / 4) {
         c->squeezed = true;
-        for (DevBuf* b : {&c->raw, &c->cone, &c->cone_tmp}) {
+        c->sweep_ne = 0;
+        for (DevBuf* b : {&c->raw, &c->cone, &c->cone_tmp, &c->sweep_blocks, &c->sweep_line, &c->box}) {
             CK(cudaFree(b->p));
             b->p = nullptr;
             b->cap = 0;
@@ -1149,8 +1209,10 @@ int trace_subset_impl(solar_gpu_context* c, const solar_gpu_scene* s, const int*
     if (bad) return fail(SOLAR_GPU_ERR_ARG, "voxel ids outside [0, %d)", N);
     DevScene ds = dev_scene(s);
     RK(padded_grid(c, s, sky, ds, st));
-    CK(launch_trace(ds, as<DirEntry>(c->dirs), D, words32, 0, n, as<int>(c->raw),
-                    as<uint32_t>(c->shadow), voxels, as<int>(c->err), st));
+    SweepTables sweep;
+    RK(sweep_tables(c, s, sky, sweep, st));
+    CK(trace_rows(sweep, ds, as<DirEntry>(c->dirs), D, words32, 0, n, as<int>(c->raw),
+                  as<uint32_t>(c->shadow), voxels, as<int>(c->err), st));
     const long long cells = (long long)n * words32;
     k_gather_shadow<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(as<uint32_t>(c->shadow), words32, voxels, n, out);
     CK(cudaGetLastError());
@@ -1249,7 +1311,8 @@ static void all_bufs(solar_gpu_context* c, DevBuf** out)
                                 &c->chunk_pos, &c->chunk_tmp, &c->mma_union, &c->mma_nch, &c->mma_cbase,
                                 &c->mma_ccnt, &c->mma_coff, &c->mma_ent, &c->mma_scale, &c->mma_over, &c->slab16,
                                 &c->dd_ovf, &c->vox_cnt, &c->vox_off, &c->vox_tmp, &c->gpad, &c->mma_sched, &c->mma_retry,
-                                &c->cone, &c->cone_tmp, &c->cone_specs};
+                                &c->cone, &c->cone_tmp, &c->cone_specs,
+                                &c->sweep_blocks, &c->sweep_line, &c->box};
     for (int i = 0; i < kNumBufs; ++i) out[i] = bufs[i];
 }
 
@@ -1279,6 +1342,7 @@ int solar_gpu_release(solar_gpu_context* c)
         b->cap = 0;
     }
     c->have_csr = c->have_barle = false;
+    c->sweep_ne = 0;
     c->N = 0;
     c->timed = false;
     c->kt_used = 0;
@@ -1331,10 +1395,12 @@ int solar_gpu_run_batch(solar_gpu_context* const* ctxs, int n, const solar_gpu_o
         solar_gpu_options ob = opts[i];
         ob.time_kernels = 0;
         c->defer_hours = true;
+        c->sweep_owner = ctxs[0];
         c->cone_shared = &ctxs[0]->cone;   // one stream: tile i's tables are built after tile i - 1 is traced
         const int rc = run_device_impl(c, &ob, &scenes[i], outs[i], st, false);
         c->defer_hours = false;
         c->cone_shared = nullptr;
+        c->sweep_owner = nullptr;
         if (rc != SOLAR_GPU_OK) return rc;
     }
     // One CUDA graph holds every tile's hour loop as a branch of its own (on

@@ -98,6 +98,23 @@ int cone_window_radius(int W, int H);
 cudaError_t launch_trace(const DevScene& s, const DirEntry* dirs, int D, int words32,
                          int voxel_offset, int chunk_count, int* raw, uint32_t* shadow,
                          const int* perm, int* err, cudaStream_t st);
+// Tracer by azimuth sweeps (sweep.cu): the same results.
+struct SweepTables {
+    const float* blocks;         // [ne y][ne x][azimuths] table blocks
+    const int* line;             // [azimuths] common cells, start masks, cz, cells
+    int ne;                      // origin classes per axis (0: no tables)
+    const float* box;            // [4][box_stride]: box maxima of the bordered grid per quadrant
+    size_t box_stride;
+};
+// Origin classes per axis that a W x H grid needs; 0 where the sweep does not apply.
+int sweep_classes(int W, int H);
+size_t sweep_block_bytes(int D, int ne);
+size_t sweep_line_bytes(int D);
+cudaError_t launch_sweep_tables(const DirEntry* dirs, int D, const SweepTables& t, cudaStream_t st);
+cudaError_t launch_box_max(const float* gpad, int W, int H, float* box, size_t stride, cudaStream_t st);
+cudaError_t launch_trace_sweep(const DevScene& s, const DirEntry* dirs, int D, int words32, int voxel_offset,
+                               int chunk_count, int* raw, uint32_t* shadow, const int* perm, const SweepTables& tabs,
+                               int* err, cudaStream_t st);
 // ovf: chunk_count + 1 ints of scratch (rows the small-table pass hands on).
 cudaError_t launch_dedupe(int chunk_count, int D, int* raw, int* counts, int* err, const int* perm, int* ovf,
                           cudaStream_t st);

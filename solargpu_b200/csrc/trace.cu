@@ -21,7 +21,7 @@
 //   * an upper ray also ends, with no hit, once it rises above every cell it
 //     can still reach (the early-exit tables of cone.cu): the reference's
 //     result with fewer steps.
-#include "sgb_internal.cuh"
+#include "dda.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -34,101 +34,6 @@ constexpr int kDirParts = 32;      // blocks per voxel block, each 1/32 of the d
 constexpr int kDedupeWarps = 4;
 constexpr int kHashSlots = 4096;   // > 2592 possible distinct hits per voxel
 constexpr int kDedupeBatch = 9;    // 2592 = 9 batches of 9 rounds of 32 directions
-
-// The tracer reads the heightmap from a copy with a one-cell border of +inf
-// ([H + 2][W + 2], cell (x, y) at (x + 1) + (y + 1) * (W + 2)).  A ray that
-// steps off the grid meets the border, whose height test is always true, so
-// the loop needs no per-axis step counts; the cell it stopped on tells a
-// border stop (no hit, as the reference's bounds check) from a hit.  Heights
-// inside the grid are the caller's, +inf included.  Each load's index is
-// clamped into the copy (one unsigned min a step), so every load stays inside
-// it whatever the float tests do; a ray never leaves the copy (the border
-// ends it first), and one that did would end on the clamped border cell and
-// return -1.  (The clamp measured 2.7% faster than a compare and branch.)
-//
-// With CONE, an upper ray also reads its direction's early-exit table
-// (cone.cu) every kBoundEvery steps: a ray above the bound of a cell it has
-// passed can hit nothing from there on (every later cell is reachable from
-// that cell), so it ends with no hit, as the reference's range test would
-// end it or as it would leave the grid.  (Reading the bound every step,
-// packed with the height, cost more in loads than the steps it saved.)
-constexpr int kBoundEvery = 12;   // steps between bound checks (4: +7.4%, 8: +1.4%, 16: +1.7% at 1024^2)
-
-__device__ __forceinline__ void dda_step(float& t, float& tMaxX, float& tMaxY, int& cell, int sx, int step_y,
-                                         const DirEntry& d)
-{
-    // one step, as selects: lanes that step on different axes stay
-    // converged (measured 119.6 -> 116.5 ms at 1024^2 against branches)
-    const bool xs = tMaxX < tMaxY;
-    t = fminf(tMaxX, tMaxY);   // = xs ? tMaxX : tMaxY (equal when not xs and equal)
-    cell += xs ? sx : step_y;
-    const float nx = __fadd_rn(tMaxX, d.dX), ny = __fadd_rn(tMaxY, d.dY);
-    tMaxX = xs ? nx : tMaxX;
-    tMaxY = xs ? tMaxY : ny;
-}
-
-template <bool UP, bool CONE>
-__device__ __forceinline__ int trace_ray(const float* __restrict__ gpad, const float* __restrict__ bound, int W,
-                                         int H, float maxz, int gx, int gy, float base_z, const DirEntry& d)
-{
-    // Cdir * 2.0f is exact, so these match the reference fused or not.
-    const float ox = __fadd_rn((float)gx, __fmul_rn(d.cx, 2.0f));
-    const float oy = __fadd_rn((float)gy, __fmul_rn(d.cy, 2.0f));
-    const float oz = __fadd_rn(base_z, __fmul_rn(d.cz, 2.0f));
-    int ix = __float2int_rd(ox);
-    int iy = __float2int_rd(oy);
-    const bool px = d.cx >= 0.0f;
-    const bool py = d.cy >= 0.0f;
-    float tMaxX = __fdiv_rn(px ? __fsub_rn(__fadd_rn((float)ix, 1.0f), ox) : __fsub_rn(ox, (float)ix), d.ax);
-    float tMaxY = __fdiv_rn(py ? __fsub_rn(__fadd_rn((float)iy, 1.0f), oy) : __fsub_rn(oy, (float)iy), d.ay);
-    const int sx = px ? 1 : -1;
-    const int sy = py ? 1 : -1;
-    // The first step checks both coordinates (the start cell, never tested,
-    // may lie up to two cells outside the grid); after it the ray is inside
-    // and moves one cell a step, so it stops on the border at the latest.
-    float t;
-    if (tMaxX < tMaxY) { t = tMaxX; ix += sx; tMaxX = __fadd_rn(tMaxX, d.dX); }
-    else               { t = tMaxY; iy += sy; tMaxY = __fadd_rn(tMaxY, d.dY); }
-    if ((unsigned)ix >= (unsigned)W || (unsigned)iy >= (unsigned)H) return 0;
-    // A start height of NaN or +inf gives no hit in the reference (every test
-    // on it is false, or true only for the height range); it would also keep
-    // the border test false, so it ends here.  -inf still stops on the border.
-    if (oz != oz || oz == __int_as_float(0x7f800000)) return 0;
-    const int Wp = W + 2;
-    const int step_y = py ? Wp : -Wp;
-    int cell = (ix + 1) + (iy + 1) * Wp;
-    const unsigned last = (unsigned)Wp * (unsigned)(H + 2) - 1u;
-    float zr;
-    // the reference tests the height range before the hit; both end the ray,
-    // and which one it was is decided once, after the loop
-    if constexpr (CONE) {
-        for (;;) {
-            // The bound of the cell the group of steps starts on also bounds
-            // every cell after it, so its load has the whole group to arrive.
-            const float b = __ldg(bound + min((unsigned)cell, last));
-#pragma unroll
-            for (int k = 0; k < kBoundEvery; ++k) {
-                zr = __fmaf_rn(d.cz, t, oz);
-                if (zr > maxz || __fsub_rn(__ldg(gpad + min((unsigned)cell, last)), zr) > 0.01f) goto stopped;
-                dda_step(t, tMaxX, tMaxY, cell, sx, step_y, d);
-            }
-            if (__fmaf_rn(d.cz, t, oz) > b) return (unsigned)cell > last ? -1 : 0;
-        }
-    } else {
-        for (;;) {
-            zr = __fmaf_rn(d.cz, t, oz);
-            if ((UP ? (zr > maxz) : (zr < 0.0f)) || __fsub_rn(__ldg(gpad + min((unsigned)cell, last)), zr) > 0.01f)
-                goto stopped;
-            dda_step(t, tMaxX, tMaxY, cell, sx, step_y, d);
-        }
-    }
-stopped:
-    if ((unsigned)cell > last) return -1;
-    if (UP ? (zr > maxz) : (zr < 0.0f)) return 0;
-    const int r = cell / Wp, q = cell - r * Wp;
-    if (q == 0 || q > W || r == 0 || r > H) return 0;   // the border: the ray left the grid
-    return (q - 1) + (r - 1) * W + 1;
-}
 
 // 16 blocks of 128 threads per SM: at most 32 registers a thread, so the SM
 // holds 64 warps of rays (measured 116.4 -> 109.7 ms at 1024^2 against 38
@@ -161,14 +66,15 @@ k_trace(DevScene s, const DirEntry* __restrict__ dirs, int D, int words32,
             const DirEntry d = dirs[g0 + k];
             // up/down and the table are the same for the whole warp (one direction at a time)
             int hit = 0;
-            if (active) {
+            Ray r;
+            if (active && ray_start(s.W, s.H, gx, gy, base_z, d, r)) {
                 if (!((d.meta >> 16) & 1))
-                    hit = trace_ray<false, false>(s.gpad, nullptr, s.W, s.H, s.maxz, gx, gy, base_z, d);
+                    hit = ray_walk<false, false>(s.gpad, nullptr, s.W, s.H, s.maxz, r, d);
                 else if (s.cone)
-                    hit = trace_ray<true, true>(s.gpad, s.cone + s.cone_stride * ((d.meta >> 17) & (kMaxConeTables - 1)),
-                                                s.W, s.H, s.maxz, gx, gy, base_z, d);
+                    hit = ray_walk<true, true>(s.gpad, s.cone + s.cone_stride * ((d.meta >> 17) & (kMaxConeTables - 1)),
+                                               s.W, s.H, s.maxz, r, d);
                 else
-                    hit = trace_ray<true, false>(s.gpad, nullptr, s.W, s.H, s.maxz, gx, gy, base_z, d);
+                    hit = ray_walk<true, false>(s.gpad, nullptr, s.W, s.H, s.maxz, r, d);
             }
             if (hit < 0) {
                 atomicOr(err, kErrTraceBounds);
