@@ -209,15 +209,15 @@ def roofline_bytes(scene, ctx_sizes, fmt, B, acc, V, entries, staged_rows=0) -> 
              every voxel.
       V = 128 (tensor cores): entries of 8 bytes (W-tile offset, fp16 hi and
              lo) per nonzero weight, the union cell id of every staged row,
-             16 B of chunk offsets per 64 rows; per voxel the visiting-order
-             index, scale, normal, shadow words and accumulator; the fp16
-             slab of the top cells read once."""
+             16 B of chunk offsets per 64 rows; per voxel the scale and its
+             sum of the hour block, read and written; the fp16 slab of the
+             top cells read once."""
     csr_entries, barle_bytes, words32 = ctx_sizes
     N, T = scene.num_total, scene.num_top
     acc_b = 16 if acc in (0, 1) else 8
     if V == 128:
         lists = entries * 8 + staged_rows * 4 + (staged_rows // 64) * 16 + 8 * (N + 1)
-        return float(lists + N * (4 + 4 + 16 + 4 * words32 + acc_b) + T * B * 2)
+        return float(lists + N * (4 + 8) + T * B * 2)
     if V == 0:
         lists = (barle_bytes if fmt == 1 else 4 * csr_entries) + 8 * (N + 1)
         return float(lists + N * (4 + 32 + 4 * words32 + acc_b) + T * B * 4)
@@ -553,6 +553,8 @@ def run_ours(args, world, rank, local, pg):
     refl_ms, refl_n = ktimes.get("reflect", (0.0, 0))
     B = args.hour_block
     V = args.group_size
+    if V == 128:   # one launch runs many hour blocks: the figures below are per hour block
+        refl_n = max(refl_n, args.steps * -(-hours_of(scene) // B))
     entries = ctx.reflection_entries()
     staged = ctx.staged_rows()
     alg = roofline_bytes(scene, (ne.value, nb.value, w.value), args.format, B, args.accumulation, V, entries, staged)

@@ -25,7 +25,8 @@ LIB = os.path.join(OUT, "libsolargpu_b200.so")
 CU_SOURCES = ["trace.cu", "sweep.cu", "cone.cu", "barle.cu", "solar.cu", "reflect.cu", "group.cu", "tile.cu", "mma.cu", "voxel.cu",
               "pipeline.cu", "noalloc.cu", "surrogate.cu"]
 CXX_SOURCES = ["sky.cpp", "cxx_api.cpp"]
-HEADERS = ["sgb_internal.cuh", "dda.cuh", "solar_math.cuh", "sky.h"]
+HEADERS = ["sgb_internal.cuh", "dda.cuh", "solar_math.cuh", "solar_pair.cuh",
+           "sky.h"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

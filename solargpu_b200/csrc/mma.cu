@@ -19,7 +19,8 @@
 //            and split as w = hi + lo, so the two fp16 MMAs carry ~22 bits of
 //            each weight; 2^e_t is kept per position for the epilogue.
 //
-// Per hour block (B = 256 hours), a persistent CTA walks its groups:
+// One launch for all hour blocks (B = 256 hours) that the slab has room for; a
+// persistent CTA walks its (hour block, group) items:
 //   producers (4 warps)  copy each chunk's 64 union rows of the fp16 slab
 //                        (I[g][256 hours], 512 B a row) with 16-byte cp.async
 //                        straight into the MN-major 128-byte-swizzled layout
@@ -27,31 +28,36 @@
 //                        stages, the copies of 3 chunks in flight -- then
 //                        fence the async proxy and arrive on the stage's
 //                        full barrier;
-//   builders (3 warps)   zero one of 3 W stages (K-major, 128-byte swizzle,
+//   builders (2 x 3 warps) zero one of 3 W stages (K-major, 128-byte swizzle,
 //                        A operand, M = voxels) and scatter the chunk's
-//                        entries, fence, arrive;
+//                        entries, fence, arrive; two teams, chunks in turn;
 //   MMA (1 thread)       tcgen05.mma kind::f16 M128 N256 K16, 4 per chunk
 //                        and tile (hi, lo), into one of two TMEM accumulators
 //                        (2 x 256 columns), tcgen05.commit frees the stage;
 //   epilogue (4 warps)   thread t = TMEM lane t = voxel t of the group: reads
-//                        its 256 hours with tcgen05.ld, adds its own direct +
-//                        diffuse (FP32, solar_I from the hour table), sums the
-//                        hours and accumulates (FP64, Kahan or plain), while
-//                        the MMAs of the next group fill the other accumulator.
+//                        its 256 hours with tcgen05.ld, sums them and adds them
+//                        to the voxel's own sum of the block (k_own_blocks),
+//                        while the MMAs of the next group fill the other
+//                        accumulator.
+// k_mma_accumulate then adds up each voxel's hour blocks (FP64, Kahan or plain).
+//
+// Bound: the MMAs.  A chunk's eight take 1024 cycles of the tensor pipe (measured
+// alone, B MN-major or K-major alike); here a chunk takes 1630 to 1800, where it
+// took 2300 to 2500 with one launch an hour block, one builder team, the own
+// terms in the epilogue and each chunk published after the wait for the stage of
+// the chunk two ahead.  Reflection of the 1024^2 city 78.5 -> 58.6 ms (1350
+// TFLOP/s of executed fp16 MMA work, the power limit in sight), 512^2 20.1 ->
+// 13.0, 160^2 2.38 -> 1.13, 64^2 1.09 -> 0.13.
 //
 // fp16 I values (RN, unbiased) and split fp16 weights keep the annual error
 // far below 1e-4 (the rounding errors of I are independent across hours).
 // Every mbarrier wait is bounded (1 s); on expiry the kernel flags
 // kErrWaitTimeout, stops issuing, lets its copies and MMAs finish (bounded)
 // and frees TMEM before it exits.
-#include "solar_math.cuh"
+#include "solar_pair.cuh"
 
 #include <atomic>
 #include <cstdlib>
-#include <functional>
-#include <queue>
-#include <utility>
-#include <vector>
 
 #include <cuda_fp16.h>
 
@@ -77,9 +83,10 @@ constexpr int kMaxDevices = 64;
 constexpr int kProducerWarps = 4;           // warps 0-3
 constexpr int kEpilogueWarp0 = 4;           // warps 4-7 (TMEM lane quarters 0-3)
 constexpr int kMmaWarp = 8;
-constexpr int kBuilderWarp0 = 9;            // warps 9-11
+constexpr int kBuilderWarp0 = 9;            // warps 9-11 and 12-14: two teams, chunks in turn
 constexpr int kBuilderWarps = 3;
-constexpr int kThreads = 12 * 32;
+constexpr int kTeams = 2;
+constexpr int kThreads = 15 * 32;
 
 // shared memory: 3 x (W hi tile | W lo tile), 4 x slab rows (the hour table
 // is read through L1: every epilogue lane reads the same entry)
@@ -281,29 +288,44 @@ k_mma_layout(int N, const long long* __restrict__ woff, const unsigned short* __
     }
 }
 
-// I[g][b] (fp16) for the top cells and the block's hours.
-constexpr int kSlabCellsPerWarp = 64;
+// slab[hour block][top cell][256 hours]: I in fp16, from hour j0 of the table on.
+// A lane owns 4 consecutive hours (their table entries stay in registers, two
+// packed pairs), a warp 128; the 8 warps of a CTA sweep the same run of cells,
+// whose normals (each component twice, as the packed pairs want them) and
+// shadow words are in shared memory.  One 256-byte store a cell and warp.  The
+// hours' entries are a cost per CTA, so large scenes take long runs (512^2,
+// 4352 hours: 64 cells 1.10 ms, 128 0.88), and small ones short runs that fill
+// the GPU.
+constexpr int kSlabWarps = 8;
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSlabWarps * 32)
 k_solar_slab16(const float4* __restrict__ geo_n, int T, const uint32_t* __restrict__ shadow, int words32,
-               const HourEntry* __restrict__ table, int j0, __half* __restrict__ slab)
+               const HourEntry* __restrict__ table, int j0, int nb, int run, uint2* __restrict__ slab)
 {
-    const int lane = threadIdx.x & 31;
-    const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int hchunks = kHours >> 5;
-    const int hc = (int)(wid % hchunks);
-    const long long g0 = (wid / hchunks) * kSlabCellsPerWarp;
-    if (g0 >= T) return;
-    const int b = hc * 32 + lane;
-    const HourEntry e = table[j0 + b];
-    const int word = e.dense >= 0 ? (e.dense >> 5) : 0;
-    const uint32_t mask = e.dense >= 0 ? (1u << (e.dense & 31)) : 0u;
-    const long long g1 = min((long long)T, g0 + kSlabCellsPerWarp);
+    extern __shared__ __align__(16) unsigned char s_run[];
+    NormalPair* s_n = reinterpret_cast<NormalPair*>(s_run);
+    uint32_t* s_shadow = reinterpret_cast<uint32_t*>(s_n + run);   // [run][words32]
+    const int lane = threadIdx.x & 31, hc = blockIdx.y * kSlabWarps + (threadIdx.x >> 5);
+    const int g0 = blockIdx.x * run, cells = min(run, T - g0);
+    for (int i = threadIdx.x; i < cells; i += kSlabWarps * 32) s_n[i] = NormalPair(__ldg(geo_n + g0 + i));
+    for (int i = threadIdx.x; i < cells * words32; i += kSlabWarps * 32)
+        s_shadow[i] = __ldg(shadow + (size_t)g0 * words32 + i);
+    __syncthreads();
+    if (hc >= nb * (kHours / 128)) return;
+    const int b = hc * 128 + 4 * lane;
+    const HourPair e = make_pair2(table[j0 + b], table[j0 + b + 1]), f = make_pair2(table[j0 + b + 2], table[j0 + b + 3]);
+    const uint32_t *e0 = s_shadow + e.word[0], *e1 = s_shadow + e.word[1], *f0 = s_shadow + f.word[0],
+                   *f1 = s_shadow + f.word[1];
+    uint2* dst = slab + (((size_t)(b / kHours) * T + g0) * kHours + b % kHours) / 4;
 #pragma unroll 4
-    for (long long g = g0; g < g1; ++g) {
-        const float4 n4 = __ldg(geo_n + g);
-        const uint32_t bit = (__ldg(shadow + g * words32 + word) & mask) ? 1u : 0u;
-        slab[g * kHours + b] = __float2half_rn(solar_I(n4, e, bit));
+    for (int g = 0; g < cells; ++g) {
+        const NormalPair n = s_n[g];
+        const int w = g * words32;
+        const float2 i0 = unpack2(solar_I2(n, e, e0[w], e1[w]));
+        const float2 i1 = unpack2(solar_I2(n, f, f0[w], f1[w]));
+        const __half2 h0 = __float22half2_rn(i0), h1 = __float22half2_rn(i1);
+        dst[(size_t)g * (kHours / 4)] =
+            make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
     }
 }
 
@@ -381,24 +403,14 @@ __device__ __forceinline__ void mma_commit(unsigned bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void accumulate(const Accum& a, int v, float x)
-{
-    if (a.mode == 0) {
-        a.f64[v] += (double)x;
-    } else if (a.mode == 1) {
-        const float y = __fsub_rn(x, a.comp[v]);
-        const float s = a.f32[v];
-        const float t = __fadd_rn(s, y);
-        a.comp[v] = __fsub_rn(__fsub_rn(t, s), y);
-        a.f32[v] = t;
-    } else {
-        a.f32[v] = __fadd_rn(a.f32[v], x);
-    }
-}
-
+// Items of a launch: (hour block, group), hour block by hour block, handed to
+// the CTAs in turn, so that the CTAs work on neighbouring groups of one or two
+// hour blocks at a time (their union rows meet in L2) and a CTA's share of the
+// uneven groups averages out over the hour blocks.  One launch for all hour
+// blocks has one ragged end instead of 17, and small scenes (45 groups at 64^2)
+// fill the GPU with several hour blocks at once.
 struct MmaTiles {
-    int N, NG;
-    const int* order;          // [N] voxel at each visiting position
+    int N, T, NG, items, rot;  // item n: hour block n / NG, group (n + rot * (n / NG)) % NG
     const long long* woff;     // [N + 1]; the union of group q starts at woff[128 q]
     const int* cells;          // union cells (descending) per group
     const int* unions;         // [NG] union size
@@ -406,68 +418,67 @@ struct MmaTiles {
     const long long* coff;     // [C + 1] first entry of each chunk
     const uint2* ent;          // entries: x = byte offset in the W tile, y = half2 (hi, lo)
     const float* scale;        // [N] 2^e per visiting position
-    const int* sched;          // [gridDim.x + 1] offsets, then the groups of each CTA
+    __device__ int block_of(int n) const { return n / NG; }
+    __device__ int group_of(int n) const
+    {
+        const int hb = n / NG;
+        return (int)((unsigned)(n - hb * NG + rot * hb) % (unsigned)NG);
+    }
 };
 
-// Walks the (group, chunk) sequence of one CTA: the CTA's groups in its
-// schedule, chunks of 64 union rows inside each group (groups with an empty
-// union have none) -- the order every role follows.
+// Walks the (item, chunk) sequence of one CTA: the CTA's items, chunks of 64
+// union rows inside each group (groups with an empty union have none) -- the
+// order every role follows.
 struct Cursor {
-    int i, iend, q, c, u;
+    int n, q, c, u;
     long long ub;   // first union cell of group q
     long long cb;   // first chunk of group q
-    __device__ Cursor(const MmaTiles& mt, int cta)
-        : i(__ldg(mt.sched + cta)), iend(__ldg(mt.sched + cta + 1)), q(0), c(0), u(0), ub(0), cb(0)
-    {
-        settle(mt);
-    }
-    __device__ bool valid() const { return i < iend; }
+    long long row0; // slab row of cell 0 in the item's hour block
+    __device__ Cursor(const MmaTiles& mt, int cta) : n(cta), q(0), c(0), u(0), ub(0), cb(0), row0(0) { settle(mt); }
+    __device__ bool valid(const MmaTiles& mt) const { return n < mt.items; }
     __device__ void settle(const MmaTiles& mt)
     {
-        const int* list = mt.sched + gridDim.x + 1;
-        for (; i < iend; ++i, c = 0) {
-            q = __ldg(list + i);
+        for (; n < mt.items; n += gridDim.x, c = 0) {
+            q = mt.group_of(n);
             u = __ldg(mt.unions + q);
             if (c * kChunk < u) break;
         }
-        if (i < iend) {
+        if (n < mt.items) {
             ub = __ldg(mt.woff + (long long)q * kGroup);
             cb = __ldg(mt.cbase + q);
+            row0 = (long long)mt.block_of(n) * mt.T;
         }
     }
     __device__ void advance(const MmaTiles& mt)
     {
         ++c;
         if (c * kChunk >= u) {
-            ++i;
+            n += gridDim.x;
             c = 0;
-            settle(mt);
+            if (n < mt.items) settle(mt);
         }
     }
     // cell of row r of the current chunk (padding rows repeat row 0: their weights are 0)
     __device__ int row_cell(const MmaTiles& mt, int r, bool want) const
     {
-        if (!want) return 0;
+        if (!want || !valid(mt)) return 0;
         const int rows = min(kChunk, u - c * kChunk);
         return __ldg(mt.cells + ub + (long long)c * kChunk + (r < rows ? r : 0));
     }
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
-k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __restrict__ geo_n,
-              const uint32_t* __restrict__ shadow, int words32, const HourEntry* __restrict__ table, int j0,
-              Accum acc, int* __restrict__ err)
+k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, float* __restrict__ sums, int* __restrict__ err)
 {
     extern __shared__ __align__(1024) unsigned char dsm[];
     __shared__ __align__(8) unsigned long long full[kBStages], emptyB[kBStages], aready[kAStages], emptyA[kAStages],
         dfull[2], dempty[2], drain;
     __shared__ unsigned s_tmem;
     __shared__ volatile int s_fail;
-    __shared__ volatile int s_bok;
+    __shared__ volatile int s_bok[kTeams];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned base = (su32(dsm) + 1023u) & ~1023u;               // stages, 1024-byte aligned
     unsigned char* gbase = dsm + (base - su32(dsm));
-    const HourEntry* tab = table + j0;
 
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&s_tmem)), "r"(512));
@@ -497,52 +508,68 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
     bool ok = true;
 
     if (warp < kProducerWarps) {
-        // ---- producers: 16 rows a warp, one 16-byte piece a lane per row; the
-        // cell ids of the next chunk load while its stage is still in use
+        // ---- producers: 16 rows a warp, one 16-byte piece a lane per row
         long long k = 0;
         const int r0 = warp * 16;
         Cursor cur(mt, blockIdx.x);
-        int my = cur.valid() ? cur.row_cell(mt, r0 + lane, lane < 16) : 0;
-        while (cur.valid() && ok) {
+        auto publish = [&](long long j) {   // chunk j's copies of this warp have landed
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(su32(&full[j % kBStages]));
+        };
+        // Cells of the next two chunks, in registers of their own (a move would wait
+        // for the load): a chunk's ids load while the chunk before it is copied.
+        int cell_a = cur.row_cell(mt, r0 + lane, lane < 16), cell_b = 0;
+        long long row_a = cur.row0, row_b = 0;
+        bool more_a = cur.valid(mt), more_b = false;
+        if (more_a) {
+            cur.advance(mt);
+            more_b = cur.valid(mt);
+            cell_b = cur.row_cell(mt, r0 + lane, lane < 16);
+            row_b = cur.row0;
+        }
+        // Copies chunk k (cells `cell`) and loads the cells of chunk k + 2.  Chunk
+        // k - 2 is published before the stage of chunk k is waited for: after it,
+        // the MMAs waited for two things in turn, the stage and the copies.
+        auto copy = [&](int& cell, long long& row0, bool& more) {
+            static_assert(kCopyLag == 2, "wait_group count below");
+            if (k >= kCopyLag) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                publish(k - kCopyLag);
+            }
             const int s = (int)(k % kBStages);
             const bool w_ok = k < kBStages || bar_wait(su32(&emptyB[s]), (unsigned)(((k / kBStages) - 1) & 1), &s_fail);
             if (!__all_sync(0xFFFFFFFFu, w_ok)) {   // the warp decides as one
                 ok = false;
-                break;
+                return;
             }
-            const int cur_cell = my;
-            const unsigned bst = base + (unsigned)(kBRegion + s * kTileB);
+            const __half* chunk = slab + row0 * kHours + lane * 8;
             const int na = lane >> 3, cc = lane & 7;
-#pragma unroll 4
+            const unsigned bst = base + (unsigned)(kBRegion + s * kTileB) + (unsigned)(na * 8192 + (r0 >> 3) * 1024);
+#pragma unroll
             for (int i = 0; i < 16; ++i) {
-                const int kr = r0 + i;
-                const int cell = __shfl_sync(0xFFFFFFFFu, cur_cell, i);
-                const __half* src = slab + (size_t)cell * kHours + lane * 8;
-                const int r8 = kr & 7;
-                const unsigned dst = bst + (unsigned)(na * 8192 + (kr >> 3) * 1024 + r8 * 128 + ((cc ^ r8) << 4));
+                const int r8 = i & 7;
+                const __half* src = chunk + (long long)__shfl_sync(0xFFFFFFFFu, cell, i) * kHours;
+                const unsigned dst = bst + (unsigned)((i >> 3) * 1024 + r8 * 128 + ((cc ^ r8) << 4));
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
-            if (k >= kCopyLag) {
-                // chunk k - 2's copies have landed (the last 2 groups may be
-                // pending): publish them to the tensor cores
-                static_assert(kCopyLag == 2, "wait_group count below");
-                asm volatile("cp.async.wait_group 2;" ::: "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) bar_arrive(su32(&full[(k - kCopyLag) % kBStages]));
-            }
-            // the next chunk's cell ids (a new group first reads its union
-            // size and base: those loads stay off the copy and arrive path)
-            cur.advance(mt);
-            my = cur.valid() ? cur.row_cell(mt, r0 + lane, lane < 16) : 0;
             ++k;
+            more = false;
+            if (cur.valid(mt)) {
+                cur.advance(mt);
+                more = cur.valid(mt);
+                cell = cur.row_cell(mt, r0 + lane, lane < 16);
+                row0 = cur.row0;
+            }
+        };
+        while (more_a && ok) {
+            copy(cell_a, row_a, more_a);
+            if (!more_b || !ok) break;
+            copy(cell_b, row_b, more_b);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0)
-            for (long long j = k >= kCopyLag ? k - kCopyLag : 0; j < k; ++j) bar_arrive(su32(&full[j % kBStages]));
+        for (long long j = k >= kCopyLag ? k - kCopyLag : 0; j < k; ++j) publish(j);
         if (!ok) {
             if (lane == 0) atomicOr(err, kErrWaitTimeout);
             s_fail = 1;
@@ -552,10 +579,8 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
         if (lane == 0) {
             long long k = 0;
             int gi = 0;
-            const int* list = mt.sched + gridDim.x + 1;
-            const int i1 = __ldg(mt.sched + blockIdx.x + 1);
-            for (int i = __ldg(mt.sched + blockIdx.x); i < i1 && ok; ++i, ++gi) {
-                const int q = __ldg(list + i);
+            for (int n = blockIdx.x; n < mt.items && ok; n += gridDim.x, ++gi) {
+                const int q = mt.group_of(n);
                 const int b = gi & 1;
                 if (gi >= 2 && !bar_wait(su32(&dempty[b]), (unsigned)(((gi >> 1) - 1) & 1), &s_fail)) {
                     ok = false;
@@ -594,18 +619,21 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
         }
         __syncwarp();
     } else if (warp >= kBuilderWarp0) {
-        // ---- builders: zero the W tiles, scatter the chunk's weights; the
-        // entries of the next chunk are loaded into registers while the
-        // builders wait for its stage
-        const int bt = threadIdx.x - kBuilderWarp0 * 32;
+        // ---- builders: zero the W tiles, scatter the chunk's weights.  Two teams
+        // take the chunks in turn, and a team loads the entries of its next chunk
+        // into registers while the other one builds: one team's chunk takes 1300
+        // cycles and more, the chunk's MMAs 1024
+        const int team = (warp - kBuilderWarp0) / kBuilderWarps;
+        const int bt = threadIdx.x - (kBuilderWarp0 + team * kBuilderWarps) * 32;
         constexpr int kBuilders = kBuilderWarps * 32;
         constexpr int kPref = 16;   // entries a thread holds ahead (8: +11%, 12: +1.6%, 20: +2%); more load at scatter
         Cursor cur(mt, blockIdx.x);
+        if (team && cur.valid(mt)) cur.advance(mt);
         uint2 pre[kPref];
         long long pe0 = 0, pe1 = 0;
         auto prefetch = [&]() {
             pe0 = pe1 = 0;
-            if (cur.valid()) {
+            if (cur.valid(mt)) {
                 const long long ci = cur.cb + cur.c;
                 pe0 = __ldg(mt.coff + ci);
                 pe1 = __ldg(mt.coff + ci + 1);
@@ -617,20 +645,20 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
             }
         };
         prefetch();
-        long long k = 0;
-        while (cur.valid() && ok) {
+        long long k = team;
+        while (cur.valid(mt) && ok) {
             const int s = (int)(k % kAStages);
-            // one thread waits for the stage; every builder takes its decision
+            // one thread waits for the stage; every builder of the team takes its decision
             if (bt == 0)
-                s_bok = (k < kAStages || bar_wait(su32(&emptyA[s]), (unsigned)(((k / kAStages) - 1) & 1), &s_fail))
-                            ? 1 : 0;
-            asm volatile("bar.sync 1, %0;" ::"r"(kBuilders) : "memory");
-            ok = s_bok != 0;
+                s_bok[team] = (k < kAStages || bar_wait(su32(&emptyA[s]), (unsigned)(((k / kAStages) - 1) & 1), &s_fail))
+                                  ? 1 : 0;
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(kBuilders) : "memory");
+            ok = s_bok[team] != 0;
             if (!ok) break;
             unsigned char* sa = gbase + (size_t)s * kAStageBytes;
             uint4* z = reinterpret_cast<uint4*>(sa);
             for (int i = bt; i < 2 * kTileA / 16; i += kBuilders) z[i] = make_uint4(0u, 0u, 0u, 0u);
-            asm volatile("bar.sync 1, %0;" ::"r"(kBuilders) : "memory");
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(kBuilders) : "memory");
 #pragma unroll
             for (int i = 0; i < kPref; ++i) {
                 if (pre[i].x != 0xFFFFFFFFu) {
@@ -644,41 +672,42 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
                 *reinterpret_cast<unsigned short*>(sa + kTileA + en.x) = (unsigned short)(en.y >> 16);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("bar.sync 1, %0;" ::"r"(kBuilders) : "memory");
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(kBuilders) : "memory");
             if (bt == 0) bar_arrive(su32(&aready[s]));
-            // the next chunk's entries load while the builders wait for its stage
-            // (after the arrive: their latency stays off the MMA's path)
+            // the team's next chunk's entries (after the arrive: their latency stays
+            // off the MMA's path)
             cur.advance(mt);
+            if (cur.valid(mt)) cur.advance(mt);
             prefetch();
-            ++k;
+            k += kTeams;
         }
         if (!ok) {
             if (bt == 0) atomicOr(err, kErrWaitTimeout);
             s_fail = 1;
         }
     } else {
-        // ---- epilogue: thread t = TMEM lane t = voxel t of the group
+        // ---- epilogue: thread t = TMEM lane t = voxel t of the group: adds the sum
+        // of its 256 hours to the voxel's own (k_own_blocks; computing that here
+        // took most of the epilogue's time, which nothing hides when a CTA has few
+        // groups)
         const int t = threadIdx.x - kEpilogueWarp0 * 32;
         const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;
         int gi = 0;
-        const int* list = mt.sched + gridDim.x + 1;
-        const int i1 = __ldg(mt.sched + blockIdx.x + 1);
-        for (int i = __ldg(mt.sched + blockIdx.x); i < i1 && ok; ++i, ++gi) {
-            const int q = __ldg(list + i);
+        for (int n = blockIdx.x; n < mt.items && ok; n += gridDim.x, ++gi) {
+            const int q = mt.group_of(n);
             const int b = gi & 1;
+            const int p = q * kGroup + t;
+            const bool valid = p < mt.N;
+            const float sc = valid ? __ldg(mt.scale + p) : 0.0f;
+            const bool any = __ldg(mt.unions + q) > 0;
             const bool w_ok = bar_wait(su32(&dfull[b]), (unsigned)((gi >> 1) & 1), &s_fail, 2 * kWaitNs);
             if (!__all_sync(0xFFFFFFFFu, w_ok)) {   // tcgen05.ld below needs the whole warp
                 ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int p = q * kGroup + t;
-            const bool valid = p < mt.N;
-            const int v = valid ? __ldg(mt.order + p) : 0;
-            const float4 n4 = __ldg(geo_n + v);
-            const float sc = valid ? __ldg(mt.scale + p) : 0.0f;
-            const bool any = mt.unions[q] > 0;
-            float sum = 0.0f;
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 2
             for (int c0 = 0; c0 < kHours; c0 += 32) {
                 unsigned r[32];
                 asm volatile(
@@ -692,17 +721,12 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
                     : "r"(tmem + lane_base + (unsigned)(b * kHours + c0)));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const HourEntry e = tab[c0 + i];
-                    const float own = solar_I(n4, e, shadow_bit(shadow, words32, v, e.dense));
-                    const float refl = any ? __uint_as_float(r[i]) * sc : 0.0f;
-                    sum += own + refl;
-                }
+                for (int i = 0; i < 32; ++i) sum[i & 3] += __uint_as_float(r[i]);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) bar_arrive(su32(&dempty[b]));
-            if (valid) accumulate(acc, v, sum);
+            if (valid && any) sums[(size_t)mt.block_of(n) * mt.N + p] += ((sum[0] + sum[1]) + (sum[2] + sum[3])) * sc;
         }
         if (!ok) {
             if (lane == 0) atomicOr(err, kErrWaitTimeout);
@@ -721,6 +745,48 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, const float4* __rest
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+    }
+}
+
+// Accumulates the hour blocks' sums (sums [nb][N] by visiting position) of every
+// voxel; first / last: the launch's blocks begin / end the year (else the
+// accumulators are read / kept).
+template <int MODE>
+__global__ void __launch_bounds__(256)
+k_mma_accumulate(const int* __restrict__ order, int N, int nb, const float* __restrict__ sums, Accum acc, bool first,
+                 bool last, float* __restrict__ out)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= N) return;
+    const int v = __ldg(order + p);
+    double a64 = 0.0;
+    float a32 = 0.0f, comp = 0.0f;
+    if (!first) {
+        if (MODE == 0) a64 = acc.f64[v];
+        else a32 = acc.f32[v];
+        if (MODE == 1) comp = acc.comp[v];
+    }
+#pragma unroll 4
+    for (int hb = 0; hb < nb; ++hb) {
+        const float x = __ldg(sums + (size_t)hb * N + p);
+        if (MODE == 0) {
+            a64 += (double)x;
+        } else if (MODE == 1) {
+            const float y = __fsub_rn(x, comp);
+            const float s = __fadd_rn(a32, y);
+            comp = __fsub_rn(__fsub_rn(s, a32), y);
+            a32 = s;
+        } else {
+            a32 = __fadd_rn(a32, x);
+        }
+    }
+    if (last) {
+        out[v] = MODE == 0 ? (float)a64 : a32;
+    } else if (MODE == 0) {
+        acc.f64[v] = a64;
+    } else {
+        acc.f32[v] = a32;
+        if (MODE == 1) acc.comp[v] = comp;
     }
 }
 
@@ -756,38 +822,6 @@ cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<bool> (&done)[kMaxDev
 }  // namespace
 
 int mma_group_count(int N) { return (N + kGroup - 1) / kGroup; }
-
-int mma_grid(int N)
-{
-    const int NG = mma_group_count(N);
-    return NG < mma_sms() ? NG : mma_sms();
-}
-
-void mma_schedule(int N, const long long* cbase, int* sched)
-{
-    const int NG = mma_group_count(N);
-    const int P = mma_grid(N);
-    if (NG <= 0 || P <= 0) return;
-    // a group costs its chunks plus about one chunk of switching (the epilogue
-    // of its accumulator, the first copies of the next group)
-    constexpr long long kGroupCost = 1;
-    std::vector<int> owner(NG), count(P, 0);
-    std::priority_queue<std::pair<long long, int>, std::vector<std::pair<long long, int>>,
-                        std::greater<std::pair<long long, int>>> load;
-    for (int b = 0; b < P; ++b) load.push({0, b});
-    for (int q = 0; q < NG; ++q) {
-        const auto top = load.top();
-        load.pop();
-        owner[q] = top.second;
-        ++count[top.second];
-        load.push({top.first + (cbase[q + 1] - cbase[q]) + kGroupCost, top.second});
-    }
-    sched[0] = 0;
-    for (int b = 0; b < P; ++b) sched[b + 1] = sched[b] + count[b];
-    std::vector<int> at(sched, sched + P);
-    int* list = sched + P + 1;
-    for (int q = 0; q < NG; ++q) list[at[owner[q]]++] = q;   // increasing within each CTA
-}
 
 cudaError_t launch_mma_union(int N, const long long* woff, int* cells, unsigned short* slots, int* unions, int* nch,
                              int* over, int* retry, cudaStream_t st)
@@ -826,30 +860,46 @@ cudaError_t launch_mma_layout(int pass, int N, const long long* woff, const unsi
 }
 
 cudaError_t launch_solar_slab16(const DevGeom& g, int T, const uint32_t* shadow, int words32, const HourEntry* table,
-                                int j0, void* slab16, cudaStream_t st)
+                                int j0, int nb, void* slab16, cudaStream_t st)
 {
-    if (T <= 0) return cudaSuccess;
-    const long long warps = ((long long)T + kSlabCellsPerWarp - 1) / kSlabCellsPerWarp * (kHours / 32);
-    k_solar_slab16<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, st>>>(g.geo_n, T, shadow, words32, table, j0,
-                                                                          static_cast<__half*>(slab16));
+    if (T <= 0 || nb <= 0) return cudaSuccess;
+    const int run = T >= 1 << 17 ? 256 : T >= 1 << 15 ? 128 : 64;
+    const size_t smem = (size_t)run * (sizeof(NormalPair) + sizeof(uint32_t) * words32);
+    if (smem > 48 * 1024) {   // up to 41 words: 54 KB
+        const cudaError_t e = cudaFuncSetAttribute(k_solar_slab16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const dim3 grid((T + run - 1) / run, (nb * (kHours / 128) + kSlabWarps - 1) / kSlabWarps);
+    k_solar_slab16<<<grid, kSlabWarps * 32, smem, st>>>(g.geo_n, T, shadow, words32, table, j0, nb, run,
+                                                        static_cast<uint2*>(slab16));
     return cudaGetLastError();
 }
 
-cudaError_t launch_reflect_mma(const void* slab16, const MmaLists& ml, const DevGeom& g, const uint32_t* shadow,
-                               int words32, const HourEntry* table, int j0, const Accum& acc, int* err,
+cudaError_t launch_reflect_mma(const void* slab16, int T, const MmaLists& ml, int nb, float* sums, int* err,
                                cudaStream_t st)
 {
     const int NG = mma_group_count(ml.N);
-    if (NG <= 0) return cudaSuccess;
+    if (NG <= 0 || nb <= 0) return cudaSuccess;
     static std::atomic<bool> attr[kMaxDevices];
     cudaError_t e = allow_smem(k_reflect_mma, (size_t)kSmemBytes, attr);
     if (e != cudaSuccess) return e;
-    if (!ml.sched) return cudaErrorInvalidValue;
-    MmaTiles mt{ml.N, NG, ml.order, ml.woff, ml.cells, ml.unions, ml.cbase, ml.coff,
-                reinterpret_cast<const uint2*>(ml.ent), ml.scale, ml.sched};
-    const int grid = mma_grid(ml.N);
-    k_reflect_mma<<<grid, kThreads, kSmemBytes, st>>>(static_cast<const __half*>(slab16), mt, g.geo_n, shadow,
-                                                       words32, table, j0, acc, err);
+    if ((long long)NG * nb > 0x7FFFFFFFLL - 4096) return cudaErrorInvalidValue;
+    const int items = NG * nb, grid = items < mma_sms() ? items : mma_sms();
+    // with a multiple of the grid's size a CTA would meet the same groups in every hour block
+    MmaTiles mt{ml.N, T, NG, items, NG % grid == 0 ? 1 : 0, ml.woff, ml.cells, ml.unions, ml.cbase, ml.coff,
+                reinterpret_cast<const uint2*>(ml.ent), ml.scale};
+    k_reflect_mma<<<grid, kThreads, kSmemBytes, st>>>(static_cast<const __half*>(slab16), mt, sums, err);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mma_accumulate(const int* order, int N, int nb, const float* sums, const Accum& acc, bool first,
+                                  bool last, float* out, cudaStream_t st)
+{
+    if (N <= 0) return cudaSuccess;
+    const unsigned grid = (unsigned)((N + 255) / 256);
+    if (acc.mode == 0) k_mma_accumulate<0><<<grid, 256, 0, st>>>(order, N, nb, sums, acc, first, last, out);
+    else if (acc.mode == 1) k_mma_accumulate<1><<<grid, 256, 0, st>>>(order, N, nb, sums, acc, first, last, out);
+    else k_mma_accumulate<2><<<grid, 256, 0, st>>>(order, N, nb, sums, acc, first, last, out);
     return cudaGetLastError();
 }
 

@@ -92,6 +92,8 @@ struct HourLoop {
     const sgb::HourEntry* tab = nullptr;
     float* slab = nullptr;
     void* slab16 = nullptr;
+    int blocks = 0;            // tensor-core kernel: hour blocks of a launch
+    float* sums = nullptr;     // and their sums
     sgb::MmaLists ml{};
     sgb::TileLists tl{};
     sgb::GroupLists gl{};
@@ -113,7 +115,7 @@ struct solar_gpu_context {
         grp_cell, grp_w, w_cnt, w_off, w_tmp, w_cell, w_val, order_first, order_inv, tile_flag, tile_pos,
         tile_start, tile_union, tile_slot, tile_rows, tile_gcnt, tile_gnch, tile_gbase, tile_tbase, tile_table,
         tile_erow, tile_ew, chunk_perm, chunk_flag, chunk_pos, chunk_tmp, mma_union, mma_nch, mma_cbase,
-        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, mma_sched, mma_retry, cone, cone_tmp, cone_specs,
+        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, hour_sums, mma_retry, cone, cone_tmp, cone_specs,
         sweep_blocks, sweep_line, box;
     int* h_scalars = nullptr;   // pinned host scratch for small read-backs
     long long mem_limit = 0;    // device bytes the buffers may hold (0: no limit)
@@ -638,17 +640,38 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
 cudaError_t enqueue_hours(solar_gpu_context* c, const HourLoop& h, cudaStream_t st)
 {
     cudaError_t le = cudaSuccess;
+    if (h.mma) {
+        const int step = h.blocks * h.B;
+        for (int j0 = 0; j0 < h.Hd && le == cudaSuccess; j0 += step) {
+            const int nb = std::min(h.blocks, (h.Hd - j0 + h.B - 1) / h.B);
+            {
+                KScope k(c, SOLAR_GPU_KT_SOLAR);
+                le = launch_solar_slab16(h.g, h.T, h.sh, h.words32, h.tab, j0, nb, h.slab16, st);
+                if (le == cudaSuccess)
+                    le = launch_own_blocks(h.g, h.order, h.N, h.sh, h.words32, h.tab, j0, nb, h.sums, st);
+            }
+            if (le == cudaSuccess) {
+                KScope k(c, SOLAR_GPU_KT_REFLECT);
+                le = launch_reflect_mma(h.slab16, h.T, h.ml, nb, h.sums, h.err, st);
+            }
+            if (le == cudaSuccess) {
+                KScope k(c, SOLAR_GPU_KT_FINALIZE);
+                le = launch_mma_accumulate(h.order, h.N, nb, h.sums, h.acc, j0 == 0, j0 + step >= h.Hd, h.out, st);
+            }
+            c->launches += 4;
+        }
+        // no daylight hour: nothing was accumulated
+        if (h.Hd <= 0) le = cudaMemsetAsync(h.out, 0, sizeof(float) * (size_t)h.N, st);
+        return le;
+    }
     for (int j0 = 0; j0 < h.Hd && le == cudaSuccess; j0 += h.B) {
         {
             KScope k(c, SOLAR_GPU_KT_SOLAR);
-            le = h.mma ? launch_solar_slab16(h.g, h.T, h.sh, h.words32, h.tab, j0, h.slab16, st)
-                       : launch_solar_slab(h.g, h.slab_rows, h.sh, h.words32, h.tab, j0, h.B, h.slab, st);
+            le = launch_solar_slab(h.g, h.slab_rows, h.sh, h.words32, h.tab, j0, h.B, h.slab, st);
         }
         if (le == cudaSuccess) {
             KScope k(c, SOLAR_GPU_KT_REFLECT);
-            if (h.mma)
-                le = launch_reflect_mma(h.slab16, h.ml, h.g, h.sh, h.words32, h.tab, j0, h.acc, h.err, st);
-            else if (h.tiled)
+            if (h.tiled)
                 le = launch_reflect_tile(h.B, h.slab, h.tl, h.order, h.acc, h.err, st);
             else if (h.group_size > 0)
                 le = launch_reflect_group(h.N, h.B, h.slab, h.gl, h.order, h.acc, st);
@@ -723,19 +746,23 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
     acc.mode = o->accumulation;
     acc.f64 = nullptr;
     acc.f32 = acc.comp = nullptr;
-    if (acc.mode == SOLAR_GPU_ACC_FP64) {
-        RK(ensure(c, c->acc_f64, sizeof(double) * (size_t)N));
-        acc.f64 = as<double>(c->acc_f64);
-        CK(cudaMemsetAsync(acc.f64, 0, sizeof(double) * (size_t)N, st));
-    } else {
-        RK(ensure(c, c->acc_f32, sizeof(float) * (size_t)N));
-        RK(ensure(c, c->acc_comp, sizeof(float) * (size_t)N));
-        acc.f32 = as<float>(c->acc_f32);
-        acc.comp = as<float>(c->acc_comp);
-        CK(cudaMemsetAsync(acc.f32, 0, sizeof(float) * (size_t)N, st));
-        CK(cudaMemsetAsync(acc.comp, 0, sizeof(float) * (size_t)N, st));
-    }
+    auto accumulators = [&](bool clear) -> int {
+        if (acc.mode == SOLAR_GPU_ACC_FP64) {
+            RK(ensure(c, c->acc_f64, sizeof(double) * (size_t)N));
+            acc.f64 = as<double>(c->acc_f64);
+            if (clear) CK(cudaMemsetAsync(acc.f64, 0, sizeof(double) * (size_t)N, st));
+        } else {
+            RK(ensure(c, c->acc_f32, sizeof(float) * (size_t)N));
+            RK(ensure(c, c->acc_comp, sizeof(float) * (size_t)N));
+            acc.f32 = as<float>(c->acc_f32);
+            acc.comp = as<float>(c->acc_comp);
+            if (clear) CK(cudaMemsetAsync(acc.f32, 0, sizeof(float) * (size_t)N, st));
+            if (clear) CK(cudaMemsetAsync(acc.comp, 0, sizeof(float) * (size_t)N, st));
+        }
+        return SOLAR_GPU_OK;
+    };
     if (B == 1) {
+        RK(accumulators(true));
         RK(ensure(c, c->hourly, sizeof(float) * (size_t)N));
         for (int j = 0; j < Hd; ++j) {
             {
@@ -844,7 +871,6 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
                         c->w_val.cap = c->tile_slot.cap = 0;
                     }
                     ml.N = N;
-                    ml.order = as<int>(c->order);
                     ml.woff = as<long long>(c->w_off);
                     ml.cells = as<int>(c->w_cell);
                     ml.unions = as<int>(c->mma_union);
@@ -852,17 +878,6 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
                     ml.coff = as<long long>(c->mma_coff);
                     ml.ent = c->mma_ent.p;
                     ml.scale = as<float>(c->mma_scale);
-                    // balanced group order over the CTAs of the hour-block kernel
-                    std::vector<long long> cb((size_t)NG + 1);
-                    CK(cudaMemcpyAsync(cb.data(), c->mma_cbase.p, sizeof(long long) * ((size_t)NG + 1),
-                                       cudaMemcpyDeviceToHost, st));
-                    CK(cudaStreamSynchronize(st));
-                    std::vector<int> sched((size_t)mma_grid(N) + 1 + NG);
-                    mma_schedule(N, cb.data(), sched.data());
-                    RK(ensure(c, c->mma_sched, sizeof(int) * sched.size()));
-                    CK(cudaMemcpyAsync(c->mma_sched.p, sched.data(), sizeof(int) * sched.size(), cudaMemcpyHostToDevice,
-                                       st));
-                    ml.sched = as<int>(c->mma_sched);
                 }
             }
             if (mma) {
@@ -999,9 +1014,34 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
         // have been released to make room (very large scenes); the tensor-core
         // kernel reads an fp16 slab of the top cells only
         float* slab = nullptr;
+        int blocks = 1;
+        float* sums = as<float>(c->w_cnt);   // one hour block's sums fit the list lengths, which are dead by now
         if (mma) {
+            // As many hour blocks a launch as the slab has room for: an eighth of the
+            // free memory (a 64th in a batch, whose contexts hold theirs at once), and one
+            // under a memory limit.  Buffers kept from an earlier call are not asked about.
+            const size_t per = 2 * (size_t)T * kMmaHours + sizeof(float) * (size_t)N;
+            const int total = std::max(1, (Hd + B - 1) / B);
+            if (c->slab16.cap >= 2 * (size_t)T * kMmaHours * total && c->hour_sums.cap >= sizeof(float) * (size_t)N * total) {
+                blocks = total;
+            } else if (total > 1 && c->mem_limit <= 0) {
+                size_t free_b = 0, total_b = 0;
+                if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+                const size_t room = (free_b + c->slab16.cap + c->hour_sums.cap) / (c->defer_hours ? 64 : 8);
+                blocks = (int)std::min<size_t>((size_t)total, std::max<size_t>(1, room / per));
+                const int launches = (total + blocks - 1) / blocks;
+                blocks = (total + launches - 1) / launches;
+                if (blocks > 1 && (ensure(c, c->slab16, 2 * (size_t)T * kMmaHours * blocks) != SOLAR_GPU_OK ||
+                                   ensure(c, c->hour_sums, sizeof(float) * (size_t)N * blocks) != SOLAR_GPU_OK)) {
+                    (void)cudaGetLastError();   // no room after all
+                    blocks = 1;
+                }
+            }
+            if (blocks > 1) sums = as<float>(c->hour_sums);
             RK(ensure(c, c->slab16, 2 * (size_t)T * kMmaHours));
+            if (blocks < total) RK(accumulators(false));
         } else {
+            RK(accumulators(true));
             RK(ensure(c, c->slab, sizeof(float) * (size_t)slab_rows * B));
             slab = as<float>(c->slab);
         }
@@ -1021,6 +1061,8 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
         h.tab = tab;
         h.slab = slab;
         h.slab16 = c->slab16.p;
+        h.blocks = blocks;
+        h.sums = sums;
         h.ml = ml;
         h.tl = tl;
         h.gl = gl;
@@ -1032,7 +1074,8 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
         if (c->defer_hours) return SOLAR_GPU_OK;   // enqueued by solar_gpu_run_batch
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        const bool use_graph = o->use_graph != 0 && !c->ktime;
+        // a few launches need no graph: capturing and instantiating one takes longer
+        const bool use_graph = o->use_graph != 0 && !c->ktime && !(mma && Hd <= 2 * blocks * B);
         if (use_graph) CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         cudaError_t le = enqueue_hours(c, h, st);
         if (use_graph) {
@@ -1076,7 +1119,7 @@ int run_device_impl(solar_gpu_context* c, const solar_gpu_options* o, const sola
         // still holds (slabs, weighted lists, group layouts) are rebuilt by
         // every run, and holding them would leave no room for Stage 1.
         CK(cudaStreamSynchronize(st));
-        DevBuf* stage23[] = {&c->slab, &c->slab16, &c->w_cnt, &c->w_off, &c->w_cell, &c->w_val, &c->grp_cell,
+        DevBuf* stage23[] = {&c->slab, &c->slab16, &c->hour_sums, &c->w_cnt, &c->w_off, &c->w_cell, &c->w_val, &c->grp_cell,
                              &c->grp_w, &c->tile_slot, &c->tile_erow, &c->tile_ew, &c->tile_table, &c->mma_ent,
                              &c->mma_ccnt, &c->mma_coff, &c->mma_scale, &c->hourly, &c->csr_ids, &c->barle_bytes};
         for (DevBuf* b : stage23) {
@@ -1310,7 +1353,7 @@ static void all_bufs(solar_gpu_context* c, DevBuf** out)
                                 &c->tile_table, &c->tile_erow, &c->tile_ew, &c->chunk_perm, &c->chunk_flag,
                                 &c->chunk_pos, &c->chunk_tmp, &c->mma_union, &c->mma_nch, &c->mma_cbase,
                                 &c->mma_ccnt, &c->mma_coff, &c->mma_ent, &c->mma_scale, &c->mma_over, &c->slab16,
-                                &c->dd_ovf, &c->vox_cnt, &c->vox_off, &c->vox_tmp, &c->gpad, &c->mma_sched, &c->mma_retry,
+                                &c->dd_ovf, &c->vox_cnt, &c->vox_off, &c->vox_tmp, &c->gpad, &c->hour_sums, &c->mma_retry,
                                 &c->cone, &c->cone_tmp, &c->cone_specs,
                                 &c->sweep_blocks, &c->sweep_line, &c->box};
     for (int i = 0; i < kNumBufs; ++i) out[i] = bufs[i];

@@ -153,6 +153,10 @@ cudaError_t launch_solar_hour(const DevGeom& g, int N, const uint32_t* shadow, i
 cudaError_t launch_solar_sum(const DevGeom& g, int N, const uint32_t* shadow, int words32,
                              const HourEntry* table, int n_hours, double* sums, cudaStream_t st);
 
+// own [nb][N]: sums of the hour blocks of 256 hours from hour j0 on, by visiting position.
+cudaError_t launch_own_blocks(const DevGeom& g, const int* order, int N, const uint32_t* shadow, int words32,
+                              const HourEntry* table, int j0, int nb, float* own, cudaStream_t st);
+
 // reflection (reflect.cu)
 struct NeighborLists {
     int format;                  // 0 = CSR, 1 = ba-RLE
@@ -250,7 +254,6 @@ cudaError_t launch_reflect_tile(int B, const float* slab, const TileLists& tl, c
 // blocks of 256, fp16 slab of the top cells.
 struct MmaLists {
     int N;
-    const int* order;          // [N] voxel at each visiting position
     const long long* woff;     // [N + 1] weighted-list offsets; the union of group q starts at woff[128 q]
     const int* cells;          // union cells per group (written over the weighted cells)
     const int* unions;         // [groups] union size
@@ -258,20 +261,11 @@ struct MmaLists {
     const long long* coff;     // [chunks + 1] first entry of each chunk
     const void* ent;           // [entries] 8 bytes: W-tile byte offset, fp16 hi, fp16 lo
     const float* scale;        // [N] per visiting position: 2^e undoing the weight scaling
-    const int* sched;          // [mma_grid + 1 + groups]: per-CTA offsets, then the groups of each CTA
 };
 constexpr int kMmaGroup = 128;
 constexpr int kMmaHours = 256;
 constexpr int kMmaChunk = 64;
 int mma_group_count(int N);
-// CTAs of the hour-block kernel for N voxels (the schedule is made for them).
-int mma_grid(int N);
-// Balanced static schedule of the groups over mma_grid(N) CTAs: in visiting
-// order, each group goes to the CTA with the least work so far (its chunks
-// plus a per-group cost), as a dynamic scheduler would hand them out, so
-// neighbouring groups still run at the same time.  cbase [groups + 1] on the
-// host; sched receives mma_grid + 1 offsets followed by the groups.
-void mma_schedule(int N, const long long* cbase, int* sched);
 // Union of each group (cells rewritten in place, slots per entry, union size
 // and chunk count per group); *over counts groups above the union cap.
 // retry: groups + 1 ints of scratch (groups the small first pass hands on).
@@ -282,11 +276,16 @@ cudaError_t launch_mma_union(int N, const long long* woff, int* cells, unsigned 
 cudaError_t launch_mma_layout(int pass, int N, const long long* woff, const unsigned short* slots, const float* wts,
                               const int* nch, const long long* cbase, int* ccnt, const long long* coff, uint2* ent,
                               float* scale, cudaStream_t st);
+// nb hour blocks from hour j0 on: slab16 [nb][T][256] fp16.
 cudaError_t launch_solar_slab16(const DevGeom& g, int T, const uint32_t* shadow, int words32, const HourEntry* table,
-                                int j0, void* slab16, cudaStream_t st);
-cudaError_t launch_reflect_mma(const void* slab16, const MmaLists& ml, const DevGeom& g, const uint32_t* shadow,
-                               int words32, const HourEntry* table, int j0, const Accum& acc, int* err,
+                                int j0, int nb, void* slab16, cudaStream_t st);
+// sums [nb][N]: adds each hour block's reflected sum, by visiting position.
+cudaError_t launch_reflect_mma(const void* slab16, int T, const MmaLists& ml, int nb, float* sums, int* err,
                                cudaStream_t st);
+// Accumulates nb hour blocks' sums; first / last: the year begins / ends with
+// them (out is written).
+cudaError_t launch_mma_accumulate(const int* order, int N, int nb, const float* sums, const Accum& acc, bool first,
+                                  bool last, float* out, cudaStream_t st);
 
 // voxelization (voxel.cu): wall voxels per cell, then the packed arrays
 // (tops [0, T), walls after them at T + off[cell] + v).

@@ -6,7 +6,7 @@
 // voxel.  Those terms depend only on the hour, so here one FP64 kernel
 // evaluates them once per daylight hour (k_hour_table); the per voxel-hour
 // work is a dot product, a shadow-bit test and three FMAs (solar_I).
-#include "solar_math.cuh"
+#include "solar_pair.cuh"
 
 namespace sgb {
 namespace {
@@ -129,22 +129,107 @@ k_solar_hour(const float4* __restrict__ geo_n, int N, const uint32_t* __restrict
     hourly[v] = solar_I(__ldg(geo_n + v), e, shadow_bit(shadow, words32, v, e.dense));
 }
 
-// sums[v] = sum over all daylight hours of I(v, h), accumulated in FP64.
-__global__ void __launch_bounds__(256)
+// ---- sums over hours ---------------------------------------------------------
+//
+// A thread sums the hours of two voxels, two hours at a time (solar_I2), with
+// the hours' pairs and the voxels' shadow words in shared memory: 11
+// instructions a voxel-hour, where a thread per voxel reading the table and its
+// shadow words through L1 took 34.
+
+constexpr int kPairs = 128;          // pairs of hours staged at a time (256 hours)
+
+__device__ __forceinline__ void stage_pairs(const HourEntry* __restrict__ table, HourPair* s_pair, int tid, int threads)
+{
+    for (int i = tid; i < kPairs; i += threads) s_pair[i] = make_pair2(table[2 * i], table[2 * i + 1]);
+}
+
+// own[hb][p] = sum of I over hour block hb (256 hours), for the voxel at
+// visiting position p.
+constexpr int kOwnThreads = 128;     // and 256 voxels
+
+__global__ void __launch_bounds__(kOwnThreads)
+k_own_blocks(const float4* __restrict__ geo_n, const int* __restrict__ order, int N, const uint32_t* __restrict__ shadow,
+             int words32, const HourEntry* __restrict__ table, float* __restrict__ own)
+{
+    extern __shared__ __align__(16) unsigned char sm[];
+    HourPair* s_pair = reinterpret_cast<HourPair*>(sm);
+    uint32_t* s_shadow = reinterpret_cast<uint32_t*>(s_pair + kPairs);   // [words32][2 kOwnThreads]
+    const int tid = threadIdx.x;
+    const int p0 = blockIdx.x * 2 * kOwnThreads + tid, p1 = p0 + kOwnThreads;
+    const int v0 = __ldg(order + min(p0, N - 1)), v1 = __ldg(order + min(p1, N - 1));
+    stage_pairs(table + (size_t)blockIdx.y * 2 * kPairs, s_pair, tid, kOwnThreads);
+    for (int w = 0; w < words32; ++w) {
+        s_shadow[w * 2 * kOwnThreads + tid] = __ldg(shadow + (size_t)v0 * words32 + w);
+        s_shadow[w * 2 * kOwnThreads + kOwnThreads + tid] = __ldg(shadow + (size_t)v1 * words32 + w);
+    }
+    __syncthreads();
+    const NormalPair n0(__ldg(geo_n + v0)), n1(__ldg(geo_n + v1));
+    f32x2 a0 = 0ull, b0 = 0ull, a1 = 0ull, b1 = 0ull;
+    const uint32_t* sh = s_shadow + tid;
+#pragma unroll 2
+    for (int i = 0; i < kPairs; i += 2) {
+        const HourPair e = s_pair[i], f = s_pair[i + 1];
+        const uint32_t *e0 = sh + e.word[0] * 2 * kOwnThreads, *e1 = sh + e.word[1] * 2 * kOwnThreads;
+        const uint32_t *f0 = sh + f.word[0] * 2 * kOwnThreads, *f1 = sh + f.word[1] * 2 * kOwnThreads;
+        a0 = add2(a0, solar_I2(n0, e, e0[0], e1[0]));
+        a1 = add2(a1, solar_I2(n1, e, e0[kOwnThreads], e1[kOwnThreads]));
+        b0 = add2(b0, solar_I2(n0, f, f0[0], f1[0]));
+        b1 = add2(b1, solar_I2(n1, f, f0[kOwnThreads], f1[kOwnThreads]));
+    }
+    const float2 s0 = unpack2(add2(a0, b0)), s1 = unpack2(add2(a1, b1));
+    float* dst = own + (size_t)blockIdx.y * N;
+    if (p0 < N) dst[p0] = s0.x + s0.y;
+    if (p1 < N) dst[p1] = s1.x + s1.y;
+}
+
+// sums[v] = sum over all daylight hours of I(v, h): FP32 over 32 hours, FP64
+// over those.  A CTA takes 64 voxels; its 4 warps take the staged hours in turn
+// (32 at a time) and their sums are added at the end, so that small scenes
+// fill the GPU.
+constexpr int kSumWarps = 4;
+
+__global__ void __launch_bounds__(kSumWarps * 32)
 k_solar_sum(const float4* __restrict__ geo_n, int N, const uint32_t* __restrict__ shadow, int words32,
             const HourEntry* __restrict__ table, int n_hours, double* __restrict__ sums)
 {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= N) return;
-    const float4 n4 = __ldg(geo_n + v);
-    double acc = 0.0;
-    float part = 0.0f;
-    for (int j = 0; j < n_hours; ++j) {
-        const HourEntry e = table[j];
-        part += solar_I(n4, e, shadow_bit(shadow, words32, v, e.dense));
-        if ((j & 31) == 31) { acc += part; part = 0.0f; }
+    extern __shared__ __align__(16) unsigned char sm[];
+    HourPair* s_pair = reinterpret_cast<HourPair*>(sm);
+    uint32_t* s_shadow = reinterpret_cast<uint32_t*>(s_pair + kPairs);   // [words32][64]
+    __shared__ double s_sum[kSumWarps][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int v = blockIdx.x * 64;
+    for (int i = threadIdx.x; i < 64 * words32; i += kSumWarps * 32)
+        s_shadow[(i % words32) * 64 + i / words32] =
+            v + i / words32 < N ? __ldg(shadow + (size_t)v * words32 + i) : 0u;
+    const NormalPair n0(__ldg(geo_n + min(v + lane, N - 1))), n1(__ldg(geo_n + min(v + 32 + lane, N - 1)));
+    const uint32_t* sh = s_shadow + lane;
+    double a0 = 0.0, a1 = 0.0;
+    for (int j = 0; j < n_hours; j += 2 * kPairs) {   // the table is padded with hours of no light
+        __syncthreads();
+        stage_pairs(table + j, s_pair, threadIdx.x, kSumWarps * 32);
+        __syncthreads();
+        for (int i = warp * 16; i < kPairs; i += kSumWarps * 16) {
+            f32x2 t0 = 0ull, t1 = 0ull;
+#pragma unroll 4
+            for (int k = 0; k < 16; ++k) {
+                const HourPair e = s_pair[i + k];
+                const uint32_t *w0 = sh + e.word[0] * 64, *w1 = sh + e.word[1] * 64;
+                t0 = add2(t0, solar_I2(n0, e, w0[0], w1[0]));
+                t1 = add2(t1, solar_I2(n1, e, w0[32], w1[32]));
+            }
+            const float2 s0 = unpack2(t0), s1 = unpack2(t1);
+            a0 += (double)s0.x + (double)s0.y;
+            a1 += (double)s1.x + (double)s1.y;
+        }
     }
-    sums[v] = acc + part;
+    s_sum[warp][lane] = a0;
+    s_sum[warp][32 + lane] = a1;
+    __syncthreads();
+    if (threadIdx.x < 64 && v + (int)threadIdx.x < N) {
+        double a = 0.0;
+        for (int w = 0; w < kSumWarps; ++w) a += s_sum[w][threadIdx.x];
+        sums[v + threadIdx.x] = a;
+    }
 }
 
 }  // namespace
@@ -185,7 +270,22 @@ cudaError_t launch_solar_hour(const DevGeom& g, int N, const uint32_t* shadow, i
 cudaError_t launch_solar_sum(const DevGeom& g, int N, const uint32_t* shadow, int words32,
                              const HourEntry* table, int n_hours, double* sums, cudaStream_t st)
 {
-    k_solar_sum<<<(N + 255) / 256, 256, 0, st>>>(g.geo_n, N, shadow, words32, table, n_hours, sums);
+    const size_t smem = sizeof(HourPair) * kPairs + sizeof(uint32_t) * 64 * (size_t)words32;
+    k_solar_sum<<<(N + 63) / 64, kSumWarps * 32, smem, st>>>(g.geo_n, N, shadow, words32, table, n_hours, sums);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_own_blocks(const DevGeom& g, const int* order, int N, const uint32_t* shadow, int words32,
+                              const HourEntry* table, int j0, int nb, float* own, cudaStream_t st)
+{
+    if (N <= 0 || nb <= 0) return cudaSuccess;
+    const size_t smem = sizeof(HourPair) * kPairs + sizeof(uint32_t) * 2 * kOwnThreads * (size_t)words32;
+    if (smem > 48 * 1024) {   // up to 41 words: 52 KB
+        const cudaError_t e = cudaFuncSetAttribute(k_own_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const dim3 grid((unsigned)((N + 2 * kOwnThreads - 1) / (2 * kOwnThreads)), nb);
+    k_own_blocks<<<grid, kOwnThreads, smem, st>>>(g.geo_n, order, N, shadow, words32, table + j0, own);
     return cudaGetLastError();
 }
 
