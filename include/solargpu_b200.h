@@ -350,6 +350,11 @@ int solar_gpu_sg_hcat(const void* a_bf16, int wa, const void* b_bf16, int wb, in
 int solar_gpu_sg_relu_grad_cols(const float* dY, int ldy, const void* H_bf16, int ldh, int rows, int cols,
                                 void* out_bf16, void* stream);
 int solar_gpu_sg_transpose_f32(const float* in, int R, int C, float* out, void* stream);
+/* A layer's weight gradient, dW[n_out][n_in] = g[rows][n_out]^T x a[rows][n_in]
+   (bf16 in, f32 out) on the tensor cores; rows, n_out and n_in multiples of 64,
+   n_out or n_in of 128, 16-byte aligned pointers.  Synchronous on `stream`. */
+int solar_gpu_sg_weight_grad(const void* g_bf16, const void* a_bf16, int rows, int n_out, int n_in, float* dW,
+                             void* stream);
 
 /* ---- encoding without device allocation -------------------------------- */
 

@@ -246,6 +246,8 @@ cudaError_t launch_tile_layout(int pass, int NG, int R, const int* start, const 
 // stall != 0 withholds the operand loads (self-test of the bounded waits).
 cudaError_t launch_gemm_bf16(const void* A, const void* B, float* C, void* Cb, const float* bias, int M, int N,
                              int K, int relu, int* err, cudaStream_t st, int stall = 0);
+// C[M][N] = X[K][M]^T x Y[K][N] (f32): M, N and K multiples of 64, M or N of 128.
+cudaError_t launch_gemm_rows(const void* X, const void* Y, float* C, int M, int N, int K, int* err, cudaStream_t st);
 // slab: [N][B] rows of every voxel (neighbor values and each voxel's own term).
 cudaError_t launch_reflect_tile(int B, const float* slab, const TileLists& tl, const int* order, const Accum& acc,
                                 int* err, cudaStream_t st);

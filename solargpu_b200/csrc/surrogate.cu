@@ -2,16 +2,16 @@
 // visibility surrogate:   C[M][N] (f32) = A[M][K] (bf16) x B[N][K]^T (bf16)
 // (+ bias[N], optional ReLU, optional bf16 copy of the result).
 //
-// One CTA of 128 threads per 128 x BN output tile (BN = 256 when N allows,
-// 64 for 64-wide outputs, else 128), K in steps of 64 through a ring of kGemmStages shared-memory
+// One CTA of 128 threads per BM x BN output tile (128 x 64, 128 or 256; 64 x 16, 32
+// or 64 where those fit one wave), K in steps of 64 through a ring of shared-memory
 // stages:
-//   * thread 0 (producer) loads each stage with tensor-map TMA, one box of
+//   * warp 0 (producer) loads each stage with tensor-map TMA, one box of
 //     64 bf16 (128 bytes) x rows per operand, 128-byte swizzle: this is the
 //     canonical K-major SWIZZLE_128B layout the tensor core reads (8-row
 //     atoms of 1024 bytes, 16-byte chunks XOR-ed with the row within the
 //     atom); completion is counted in bytes on the stage's full mbarrier;
-//   * thread 32 (MMA issuer) waits for a stage, issues 4 tcgen05.mma (K = 16
-//     each, 32 bytes further along the swizzled rows; M = 128, N = BN, f32
+//   * warp 1 (MMA) waits for a stage, issues 4 tcgen05.mma a K step (K = 16
+//     each, 32 bytes further along the swizzled rows; M = BM, N = BN, f32
 //     accumulator in BN TMEM columns) and tcgen05.commit frees the stage
 //     (empty mbarrier) when they complete; a last commit signals the
 //     epilogue;
@@ -39,15 +39,24 @@ constexpr int kGemmThreads = 128;
 constexpr int kGemmStages = 4;
 constexpr unsigned long long kGemmWaitNs = 1000000000ull;   // 1 s
 
-template <int BN>
+// ROWS: the product sums over the rows of both operands (C = X^T Y, X [K][M],
+// Y [K][N]): tiles are [64 rows][BM or BN columns], M and N contiguous.
+template <int BM, int BN, bool ROWS = false>
 struct GemmShape {
-    static constexpr int kStageA = kTm * kTk * 2, kStageB = BN * kTk * 2;     // 16 KB, 16/32 KB
-    static constexpr int kStage = kStageA + kStageB;
-    static constexpr int kSmem = kGemmStages * kStage + 1024;              // + alignment slack
+    static constexpr int kStageA = BM * kTk * 2, kStageB = BN * kTk * 2;
+    static constexpr int kStage = kStageA + kStageB;                       // one K step
+    // tiles of 64 rows: 4 K steps a stage (a wait, a vote and a commit for 16 MMAs), and
+    // as many stages as an SM's shared memory holds
+    static constexpr int kSteps = BM == kTm ? 1 : 4;
+    static constexpr int kStages = BM == kTm ? kGemmStages : 200 * 1024 / (kSteps * kStage);
+    static constexpr int kSmem = kStages * kSteps * kStage + 1024;   // + alignment slack
+    static constexpr int kTmemCols = BN < 32 ? 32 : BN;
     // Instruction descriptor, kind::f16: f32 accumulator, bf16 A and B,
-    // both K-major, N = BN, M = 128.
-    static constexpr unsigned kIdesc =
-        (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(kTm >> 4) << 24);
+    // both K-major (ROWS: both MN-major), N = BN, M = BM.
+    static constexpr unsigned kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (ROWS ? 3u << 15 : 0u) |
+                                       ((unsigned)(BN >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
+    // from one K = 16 to the next within a step, in the descriptors' 16-byte units
+    static constexpr unsigned kNextA = ROWS ? BM * 2 : 2, kNextB = ROWS ? BN * 2 : 2;
 };
 
 __device__ __forceinline__ unsigned s_u32(const void* p)
@@ -94,6 +103,17 @@ __device__ __forceinline__ unsigned long long smem_desc_sw128(unsigned addr)
            (1ull << 46) | (2ull << 61);
 }
 
+// The same for an MN-major tile of `width` elements (16, 32 or 64: rows of 32, 64 or
+// 128 bytes, swizzled over as many): 8 K rows an atom, the next 8 behind it; the
+// tile is one atom wide, so the other offset is unused.
+template <int WIDTH>
+__device__ __forceinline__ unsigned long long smem_desc_rows(unsigned addr)
+{
+    constexpr unsigned long long type = WIDTH == 64 ? 2 : WIDTH == 32 ? 4 : 6;
+    return (unsigned long long)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((unsigned long long)(WIDTH * 16 >> 4) << 32) |
+           (1ull << 46) | (type << 61);
+}
+
 __device__ __forceinline__ void tma_box(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar)
 {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -101,30 +121,68 @@ __device__ __forceinline__ void tma_box(unsigned dst, const CUtensorMap* map, in
                  : "memory");
 }
 
-template <int BN>
+// The role warps run their loops as whole warps, with one elected lane for the
+// instructions of a single thread: stage addresses and descriptors stay in the
+// uniform registers those instructions take, where a loop of one lane moved each
+// there anew, and the warp's other lanes polled the last barrier in turn with it.
+// A K step of a lone 128 x 64 tile took 359 ns that way (33 of them a MMA), 227
+// this way; tiles of 64 x 16 with 4 steps a stage take 83.
+__device__ __forceinline__ bool elect_one()
+{
+    unsigned p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+__device__ __forceinline__ bool warp_wait(unsigned bar, unsigned parity, const volatile int* fail)
+{
+    return __all_sync(0xFFFFFFFFu, wait_parity(bar, parity, fail));
+}
+
+// One K step of 64 through shared-memory descriptors da, db (4 MMAs), by one thread.
+template <typename S>
+__device__ __forceinline__ void mma_step(unsigned tmem, unsigned long long da, unsigned long long db, bool first)
+{
+#pragma unroll
+    for (int j = 0; j < kTk / 16; ++j) {
+        const unsigned acc = (!first || j > 0) ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+            ::"r"(tmem), "l"(da + S::kNextA * j), "l"(db + S::kNextB * j), "r"(S::kIdesc), "r"(acc), "r"(0), "r"(0), "r"(0), "r"(0));
+    }
+}
+
+__device__ __forceinline__ void mma_commit(unsigned bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+template <int BM, int BN, bool ROWS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 k_gemm_bf16(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
             float* __restrict__ C, __nv_bfloat16* __restrict__ Cb, const float* __restrict__ bias, int M, int N, int K,
             int relu, int* __restrict__ err, int stall)
 {
+    using S = GemmShape<BM, BN, ROWS>;
     extern __shared__ __align__(1024) unsigned char gsm[];
-    __shared__ __align__(8) unsigned long long full[kGemmStages], empty[kGemmStages], done;
+    __shared__ __align__(8) unsigned long long full[S::kStages], empty[S::kStages], done;
     __shared__ unsigned tmem_base;
     __shared__ volatile int s_fail;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    using S = GemmShape<BN>;
-    const int m0 = blockIdx.y * kTm, n0 = blockIdx.x * BN;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     // 1024-byte aligned stage ring
     const unsigned base = (s_u32(gsm) + 1023u) & ~1023u;
-    const int nk = K / kTk;
+    const int nk = K / kTk, loads = (nk + S::kSteps - 1) / S::kSteps;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(&tmem_base)),
-                     "r"(BN));
+                     "r"(S::kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kGemmStages; ++s) {
+        for (int s = 0; s < S::kStages; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s_u32(&full[s])), "r"(1));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s_u32(&empty[s])), "r"(1));
         }
@@ -138,54 +196,56 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
     const unsigned tmem = tmem_base;
 
     int issued = 0;   // producer: stages loaded
-    if (threadIdx.x == 0) {
-        // ---- producer (stall: issues nothing, so the MMA thread's bounded
+    if (warp == 0) {
+        // ---- producer (stall: issues nothing, so the MMA warp's bounded
         // wait runs out; the self-test of the error path)
-        for (int k = 0; k < (stall ? 0 : nk); ++k) {
-            const int s = k % kGemmStages;
-            if (k >= kGemmStages &&
-                !wait_parity(s_u32(&empty[s]), (unsigned)(((k / kGemmStages) - 1) & 1), &s_fail)) {
+        const int n = stall ? 0 : loads;
+        for (int s = 0, round = 0; issued < n; ++issued) {
+            if (round > 0 && !warp_wait(s_u32(&empty[s]), (unsigned)((round - 1) & 1), &s_fail)) {
                 s_fail = 1;
                 break;
             }
-            const unsigned sa = base + (unsigned)(s * S::kStage), sb = sa + S::kStageA;
-            const unsigned fb = s_u32(&full[s]);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
-                         "r"((unsigned)S::kStage) : "memory");
-            tma_box(sa, &mapA, k * kTk, m0, fb);
-            tma_box(sb, &mapB, k * kTk, n0, fb);
-            ++issued;
+            if (elect_one()) {
+                const int k0 = issued * S::kSteps, steps = min(S::kSteps, nk - k0);
+                const unsigned sa = base + (unsigned)(s * S::kSteps * S::kStage), fb = s_u32(&full[s]);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
+                             "r"((unsigned)(steps * S::kStage)) : "memory");
+#pragma unroll
+                for (int j = 0; j < S::kSteps; ++j) {
+                    if (j >= steps) break;
+                    const unsigned da = sa + (unsigned)(j * S::kStage), db = da + S::kStageA;
+                    const int kk = (k0 + j) * kTk;
+                    tma_box(da, &mapA, ROWS ? m0 : kk, ROWS ? kk : m0, fb);
+                    tma_box(db, &mapB, ROWS ? n0 : kk, ROWS ? kk : n0, fb);
+                }
+            }
+            if (++s == S::kStages) { s = 0; ++round; }
         }
-    } else if (threadIdx.x == 32) {
-        // ---- MMA issuer
-        int k = 0;
-        for (; k < nk; ++k) {
-            const int s = k % kGemmStages;
-            if (!wait_parity(s_u32(&full[s]), (unsigned)((k / kGemmStages) & 1), &s_fail)) {
+    } else if (warp == 1) {
+        // ---- MMA
+        const unsigned sb = base + S::kStageA;
+        const unsigned long long da = ROWS ? smem_desc_rows<64>(base) : smem_desc_sw128(base);
+        const unsigned long long db = ROWS ? smem_desc_rows<BN>(sb) : smem_desc_sw128(sb);
+        for (int k = 0, s = 0, round = 0; k < nk; k += S::kSteps) {
+            if (!warp_wait(s_u32(&full[s]), (unsigned)(round & 1), &s_fail)) {
                 s_fail = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned sa = base + (unsigned)(s * S::kStage), sb = sa + S::kStageA;
+            if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < kTk / 16; ++j) {
-                const unsigned long long da = smem_desc_sw128(sa + 32u * j);
-                const unsigned long long db = smem_desc_sw128(sb + 32u * j);
-                const unsigned acc = (k > 0 || j > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                    ::"r"(tmem), "l"(da), "l"(db), "r"(S::kIdesc), "r"(acc), "r"(0), "r"(0), "r"(0), "r"(0));
+                for (int j = 0; j < S::kSteps; ++j) {
+                    if (k + j >= nk) break;
+                    const unsigned at = (unsigned)((s * S::kSteps + j) * (S::kStage >> 4));
+                    mma_step<S>(tmem, da + at, db + at, k + j == 0);
+                }
+                mma_commit(s_u32(&empty[s]));   // the stage is free once these MMAs have read it
             }
-            // the stage is free once these MMAs have read it
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(s_u32(&empty[s])) : "memory");
+            if (++s == S::kStages) { s = 0; ++round; }
         }
-        // all MMAs issued so far complete -> epilogue
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                     ::"r"(s_u32(&done)) : "memory");
+        if (elect_one()) mma_commit(s_u32(&done));   // all MMAs issued so far complete -> epilogue
     }
+    __syncwarp();
     // everyone: the accumulator is ready (or the run failed)
     // longer than the pipeline's waits, so a failed pipeline always signals first
     if (!wait_parity(s_u32(&done), 0u, nullptr, 2 * kGemmWaitNs)) s_fail = 1;
@@ -194,8 +254,10 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (ok) {
-        // epilogue: warp w holds rows 32w.. of the tile (TMEM lanes 32w..)
-        const int row = m0 + 32 * warp + lane;
+        // epilogue: warp w holds rows 32w.. of the tile (TMEM lanes 32w..); of a
+        // 64-row tile rows 16w.., in the first 16 of its lanes
+        const int row = m0 + BM / 4 * warp + lane;
+        const bool mine = lane < BM / 4;
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 8) {
             unsigned r[8];
@@ -211,28 +273,28 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                 v[j] = __uint_as_float(r[j]) + (bias ? bias[n0 + c0 + j] : 0.0f);
                 if (relu) v[j] = fmaxf(v[j], 0.0f);
             }
-            if (C) {
+            if (C && mine) {
                 float4* dst = reinterpret_cast<float4*>(C + (size_t)row * N + n0 + c0);
                 dst[0] = make_float4(v[0], v[1], v[2], v[3]);
                 dst[1] = make_float4(v[4], v[5], v[6], v[7]);
             }
-            if (Cb) {
+            if (Cb && mine) {
                 __nv_bfloat162 h[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
                 *reinterpret_cast<uint4*>(Cb + (size_t)row * N + n0 + c0) = *reinterpret_cast<uint4*>(h);
             }
         }
-    } else if (threadIdx.x == 0) {
-        atomicOr(err, kErrWaitTimeout);
-        // let the TMA copies this thread issued land before the CTA exits
-        for (int k = (issued > kGemmStages ? issued - kGemmStages : 0); k < issued; ++k)
-            wait_parity(s_u32(&full[k % kGemmStages]), (unsigned)((k / kGemmStages) & 1), nullptr);
+    } else if (warp == 0) {
+        if (lane == 0) atomicOr(err, kErrWaitTimeout);
+        // let the TMA copies this warp issued land before the CTA exits
+        for (int k = (issued > S::kStages ? issued - S::kStages : 0); k < issued; ++k)
+            wait_parity(s_u32(&full[k % S::kStages]), (unsigned)((k / S::kStages) & 1), nullptr);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::kTmemCols));
 }
 
 // Persistent form for grids of more than one wave: one CTA per SM walks the
@@ -244,10 +306,15 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
 //     accumulator's full barrier;
 //   * warps 2..5 are the epilogue: warp w reads TMEM lanes 32 (w % 4) ..
 //     (rows of the tile), stores them and arrives on the accumulator's empty
-//     barrier, so tile i's epilogue overlaps tile i + 1's MMAs.
+//     barrier, so tile i's epilogue overlaps tile i + 1's MMAs.  A product of
+//     few K steps is bound by these stores: [2^18 x 1024], K = 64 (1.07 GB of
+//     f32) took 442 us with each lane storing 32 bytes of its own row, 187 with
+//     128-byte rows from shared memory (5.7 TB/s).
 // Every wait is bounded and checks a shared failure flag, so all roles leave
 // their loops once one wait runs out; a last commit lets the MMAs in flight
 // finish and the TMA thread waits for its copies before TMEM is freed.
+constexpr int kStagePitch = 36;   // floats a row of an epilogue warp's 32 x 32 stage (16-byte rows, spread over the banks)
+constexpr int kPersStage = 4 * 32 * kStagePitch * 4;
 constexpr int kPersThreads = 192;
 
 template <int BN>
@@ -261,8 +328,9 @@ k_gemm_bf16_pers(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     __shared__ unsigned tmem_base;
     __shared__ volatile int s_fail;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    using S = GemmShape<BN>;
+    using S = GemmShape<kTm, BN>;
     const unsigned base = (s_u32(gsm) + 1023u) & ~1023u;
+    float* const stage = reinterpret_cast<float*>(gsm + (base - s_u32(gsm)) + kGemmStages * S::kStage);
     const int nk = K / kTk;
     const int ntn = N / BN;
     const int ntiles = (M / kTm) * ntn;
@@ -370,32 +438,40 @@ k_gemm_bf16_pers(const __grid_constant__ CUtensorMap mapA, const __grid_constant
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int t = (int)blockIdx.x + i * (int)gridDim.x;
             const int m0 = (t / ntn) * kTm, n0 = (t % ntn) * BN;
-            const int row = m0 + 32 * q + lane;
+            // 32 columns at a time through shared memory: a lane reads a row of the
+            // accumulator, but a store of the warp covers 4 rows of 128 bytes
+            float* const mine = stage + q * 32 * kStagePitch;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 8) {
-                unsigned r[8];
+            for (int c0 = 0; c0 < BN; c0 += 32) {
+                unsigned r[32];
                 const unsigned taddr = tmem + ((unsigned)(32 * q) << 16) + (unsigned)(b * BN + c0);
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                               "=r"(r[7])
-                             : "r"(taddr));
+#pragma unroll
+                for (int h = 0; h < 32; h += 8)
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                                 : "=r"(r[h]), "=r"(r[h + 1]), "=r"(r[h + 2]), "=r"(r[h + 3]), "=r"(r[h + 4]),
+                                   "=r"(r[h + 5]), "=r"(r[h + 6]), "=r"(r[h + 7])
+                                 : "r"(taddr + (unsigned)h));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float v[8];
+                __syncwarp();   // the stage's last readers are done
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    v[j] = __uint_as_float(r[j]) + (bias ? bias[n0 + c0 + j] : 0.0f);
-                    if (relu) v[j] = fmaxf(v[j], 0.0f);
-                }
-                if (C) {
-                    float4* dst = reinterpret_cast<float4*>(C + (size_t)row * N + n0 + c0);
-                    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-                    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-                }
-                if (Cb) {
-                    __nv_bfloat162 h[4];
+                for (int h = 0; h < 32; h += 4)
+                    *reinterpret_cast<uint4*>(mine + lane * kStagePitch + h) = make_uint4(r[h], r[h + 1], r[h + 2], r[h + 3]);
+                __syncwarp();
+                const int c = c0 + 4 * (lane & 7);
+                float4 add = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (bias) add = make_float4(bias[n0 + c], bias[n0 + c + 1], bias[n0 + c + 2], bias[n0 + c + 3]);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                    *reinterpret_cast<uint4*>(Cb + (size_t)row * N + n0 + c0) = *reinterpret_cast<uint4*>(h);
+                for (int h = 0; h < 32; h += 4) {
+                    const int rr = h + (lane >> 3);
+                    float4 v = *reinterpret_cast<const float4*>(mine + rr * kStagePitch + 4 * (lane & 7));
+                    v = make_float4(v.x + add.x, v.y + add.y, v.z + add.z, v.w + add.w);
+                    if (relu) v = make_float4(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, 0.0f));
+                    const size_t at = (size_t)(m0 + 32 * q + rr) * N + n0 + c;
+                    if (C) *reinterpret_cast<float4*>(C + at) = v;
+                    if (Cb) {
+                        const __nv_bfloat162 e[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+                        *reinterpret_cast<uint2*>(Cb + at) = *reinterpret_cast<const uint2*>(e);
+                    }
                 }
             }
             // the accumulator may be overwritten once all four warps have read it
@@ -405,6 +481,7 @@ k_gemm_bf16_pers(const __grid_constant__ CUtensorMap mapA, const __grid_constant
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s_u32(&tempty[b])) : "memory");
         }
     }
+    __syncwarp();   // the role warps' other lanes do not poll beside their lane 0
     // every MMA issued has completed (or the wait gave up after twice the pipeline's limit)
     if (!wait_parity(s_u32(&done), 0u, nullptr, 2 * kGemmWaitNs)) s_fail = 1;
     __syncthreads();
@@ -496,33 +573,90 @@ __global__ void k_sg_relu_grad(const float* __restrict__ dY, const __nv_bfloat16
         dX[t] = __float2bfloat16_rn(__bfloat162float(H[t]) > 0.0f ? dY[t] : 0.0f);
 }
 
-// out[c][r] = in[r][c] (bf16, 32 x 32 tiles through shared memory).
-__global__ void k_sg_transpose(const __nv_bfloat16* __restrict__ in, int R, int C, __nv_bfloat16* __restrict__ out)
+// out[c][r] = in[r][c] (bf16).  VEC: 64 x 64 tiles, 16-byte loads and stores (R
+// and C multiples of 8, pointers 16-byte aligned): 128-byte rows both ways, where
+// 32 x 32 tiles of 2-byte accesses moved 64 bytes a row.
+constexpr int kTrTile = 64;
+
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+k_sg_transpose(const __nv_bfloat16* __restrict__ in, int R, int C, __nv_bfloat16* __restrict__ out)
 {
-    __shared__ __nv_bfloat16 t[32][33];
-    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;   // row tiles on x (up to 2^31 - 1)
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int r = r0 + k, c = c0 + threadIdx.x;
-        if (r < R && c < C) t[k][threadIdx.x] = in[(size_t)r * C + c];
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c = c0 + k, r = r0 + threadIdx.x;
-        if (r < R && c < C) out[(size_t)c * R + r] = t[threadIdx.x][k];
+    __shared__ __nv_bfloat16 t[kTrTile][kTrTile + 2];   // rows 33 words apart: no conflicts down a column
+    const long long r0 = (long long)blockIdx.x * kTrTile;   // row tiles on x (up to 2^31 - 1)
+    const int c0 = blockIdx.y * kTrTile;
+    if (VEC) {
+        for (int i = threadIdx.x; i < kTrTile * 8; i += 256) {
+            const int k = i >> 3, c8 = (i & 7) * 8;
+            if (r0 + k < R && c0 + c8 < C) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(in + (size_t)(r0 + k) * C + c0 + c8));
+                unsigned* d = reinterpret_cast<unsigned*>(&t[k][c8]);
+                d[0] = v.x;
+                d[1] = v.y;
+                d[2] = v.z;
+                d[3] = v.w;
+            }
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTrTile * 8; i += 256) {
+            const int c = i >> 3, r8 = (i & 7) * 8;
+            if (r0 + r8 < R && c0 + c < C) {
+                __align__(16) __nv_bfloat16 e[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) e[q] = t[r8 + q][c];
+                *reinterpret_cast<uint4*>(out + (size_t)(c0 + c) * R + r0 + r8) = *reinterpret_cast<const uint4*>(e);
+            }
+        }
+    } else {
+        for (int i = threadIdx.x; i < kTrTile * kTrTile; i += 256) {
+            const int k = i / kTrTile, c = i % kTrTile;
+            if (r0 + k < R && c0 + c < C) t[k][c] = in[(size_t)(r0 + k) * C + c0 + c];
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTrTile * kTrTile; i += 256) {
+            const int c = i / kTrTile, k = i % kTrTile;
+            if (r0 + k < R && c0 + c < C) out[(size_t)(c0 + c) * R + r0 + k] = t[k][c];
+        }
     }
 }
 
-// out[c] += sum over the rows r0 .. r0 + rows_per_block of in[r][c] (bias
-// gradients; out zeroed first, one atomic add per column and block).
-__global__ void k_sg_colsum(const __nv_bfloat16* __restrict__ in, int R, int C, int rows_per_block,
-                            float* __restrict__ out)
+// out[c] += sum over a block's rows of in[r][c] (bias gradients; out zeroed
+// first, one atomic add per column and block).  VEC: a thread reads 8 columns of
+// a row (C a multiple of 8, in 16-byte aligned), so a row of 64 channels is 8
+// threads' and a block reads 32 rows at once; else a thread reads one column.
+constexpr int kSumGroups = 64;   // column groups a block covers; its other threads take further rows
+
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+k_sg_colsum(const __nv_bfloat16* __restrict__ in, int R, int C, int rows_per_block, float* __restrict__ out)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
-    const int r0 = blockIdx.y * rows_per_block, r1 = min(R, r0 + rows_per_block);
-    float s = 0.0f;
-    for (int r = r0; r < r1; ++r) s += __bfloat162float(in[(size_t)r * C + c]);
-    atomicAdd(out + c, s);
+    constexpr int L = VEC ? 8 : 1;
+    __shared__ float s_sum[L][256];
+    const int groups = C / L, g0 = blockIdx.x * kSumGroups, ng = min(kSumGroups, groups - g0);
+    const int lanes = 256 / ng, lane = (int)threadIdx.x / ng, g = g0 + (int)threadIdx.x % ng;
+    const long long r0 = (long long)blockIdx.y * rows_per_block, r1 = min((long long)R, r0 + rows_per_block);
+    float s[L] = {};
+    if (lane < lanes) {
+#pragma unroll 4
+        for (long long r = r0 + lane; r < r1; r += lanes) {
+            if (VEC) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(in + r * C) + g);
+                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+#pragma unroll
+                for (int q = 0; q < L; ++q) s[q] += __bfloat162float(e[q]);
+            } else {
+                s[0] += __bfloat162float(in[r * C + g]);
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < L; ++q) s_sum[q][threadIdx.x] = s[q];
+    __syncthreads();
+    for (int i = threadIdx.x; i < ng * L; i += 256) {
+        float x = 0.0f;
+        for (int l = 0; l < lanes; ++l) x += s_sum[i % L][l * ng + i / L];
+        atomicAdd(out + g0 * L + i, x);
+    }
 }
 
 // Adam on FP32 master parameters; the bf16 copy feeds the GEMMs.
@@ -600,16 +734,23 @@ __global__ void k_sg_image(const float* __restrict__ grid, const float* __restri
 // cols[(b * Ho + oy) * Wo + ox][(ky * 4 + kx) * Cin + c] = X[b][2oy-1+ky][2ox-1+kx][c]
 // (0 outside the image), columns 16 * Cin .. Kp - 1 zero.  One thread per 8
 // consecutive columns (Cin % 8 == 0: one 16-byte load and store).
+constexpr long long kIndex32 = 1LL << 31;   // thread counts up to here: 32-bit indices (a grid stride more does not wrap)
+
+// U: the index type, unsigned where the thread count fits (a 64-bit division is
+// some 100 instructions, and each group needs four).  With 2 channels (the image
+// itself) a group of 8 columns is one row of the kernel: four 4-byte loads
+// where X is aligned for them.
+template <typename U>
 __global__ void k_sg_im2col(const __nv_bfloat16* __restrict__ X, int B, int Hi, int Wi, int Cin, int Kp,
                             __nv_bfloat16* __restrict__ cols)
 {
-    const int Ho = Hi / 2, Wo = Wi / 2, K = 16 * Cin, g8 = Kp / 8;
-    const long long n = (long long)B * Ho * Wo * g8;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const long long row = t / g8;
-        const int k0 = (int)(t % g8) * 8;
-        const int ox = (int)(row % Wo), oy = (int)((row / Wo) % Ho);
-        const long long b = row / ((long long)Wo * Ho);
+    const unsigned Ho = Hi / 2, Wo = Wi / 2, g8 = Kp / 8;
+    const int K = 16 * Cin;
+    const U n = (U)B * Ho * Wo * g8;
+    for (U t = (U)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (U)gridDim.x * blockDim.x) {
+        const U row = t / g8, line = row / Wo, b = line / Ho;
+        const int k0 = (int)(t - row * g8) * 8;
+        const int ox = (int)(row - line * Wo), oy = (int)(line - b * Ho);
         uint4 out = make_uint4(0u, 0u, 0u, 0u);
         if (Cin % 8 == 0) {
             if (k0 < K) {
@@ -618,8 +759,17 @@ __global__ void k_sg_im2col(const __nv_bfloat16* __restrict__ X, int B, int Hi, 
                 if (y >= 0 && y < Hi && x >= 0 && x < Wi)
                     out = *reinterpret_cast<const uint4*>(X + (((size_t)b * Hi + y) * Wi + x) * Cin + c);
             }
+        } else if (Cin == 2 && (reinterpret_cast<uintptr_t>(X) & 3) == 0) {
+            const int y = 2 * oy - 1 + k0 / 8;
+            if (k0 < K && y >= 0 && y < Hi) {
+                const unsigned* p = reinterpret_cast<const unsigned*>(X) + ((size_t)b * Hi + y) * Wi + 2 * ox;
+                if (ox > 0) out.x = __ldg(p - 1);
+                out.y = __ldg(p);
+                out.z = __ldg(p + 1);
+                if (2 * ox + 2 < Wi) out.w = __ldg(p + 2);
+            }
         } else {
-            __nv_bfloat16 e[8];
+            __align__(16) __nv_bfloat16 e[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int k = k0 + q;
@@ -632,7 +782,7 @@ __global__ void k_sg_im2col(const __nv_bfloat16* __restrict__ X, int B, int Hi, 
             }
             out = *reinterpret_cast<uint4*>(e);
         }
-        *reinterpret_cast<uint4*>(cols + row * Kp + k0) = out;
+        *reinterpret_cast<uint4*>(cols + (size_t)row * Kp + k0) = out;
     }
 }
 
@@ -640,16 +790,17 @@ __global__ void k_sg_im2col(const __nv_bfloat16* __restrict__ X, int B, int Hi, 
 // g[b][y][x][c] = bf16( (X[b][y][x][c] > 0) * sum over the (<= 2 x 2) output
 // positions whose 4 x 4 window covers (y, x) of dcols[row][tap * Cin + c] ).
 // One thread per 8 channels (Cin % 8 == 0).
+template <typename U>
 __global__ void k_sg_col2im_relu(const float* __restrict__ dcols, const __nv_bfloat16* __restrict__ X, int B, int Hi,
                                  int Wi, int Cin, int Kp, __nv_bfloat16* __restrict__ g)
 {
-    const int Ho = Hi / 2, Wo = Wi / 2, g8 = Cin / 8;
-    const long long n = (long long)B * Hi * Wi * g8;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const long long pix = t / g8;
-        const int c0 = (int)(t % g8) * 8;
-        const int x = (int)(pix % Wi), y = (int)((pix / Wi) % Hi);
-        const long long b = pix / ((long long)Wi * Hi);
+    const int Ho = Hi / 2, Wo = Wi / 2;
+    const unsigned g8 = Cin / 8;
+    const U n = (U)B * Hi * Wi * g8;
+    for (U t = (U)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (U)gridDim.x * blockDim.x) {
+        const U pix = t / g8, line = pix / (unsigned)Wi, b = line / (unsigned)Hi;
+        const int c0 = (int)(t - pix * g8) * 8;
+        const int x = (int)(pix - line * Wi), y = (int)(line - b * Hi);
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
@@ -737,81 +888,123 @@ EncodeTiled encode_fn()
     return fn;
 }
 
-// Row-major [rows][K] bf16 matrix, boxes of 64 elements (128 bytes) x box_rows
-// rows with 128-byte swizzle.
-bool make_map(CUtensorMap* map, const void* ptr, int rows, int K, int box_rows)
+// Row-major [rows][cols] bf16 matrix, boxes of box_cols elements (64, 32 or 16: 128,
+// 64 or 32 bytes, swizzled over as many) x box_rows rows.
+bool make_map(CUtensorMap* map, const void* ptr, int rows, int cols, int box_rows, int box_cols = kTk)
 {
     EncodeTiled fn = encode_fn();
     if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kTk, (cuuint32_t)box_rows};
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    const CUtensorMapSwizzle swizzle = box_cols == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                                       : box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                        : CU_TENSOR_MAP_SWIZZLE_32B;
     const cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
-cudaError_t launch_gemm_tiles(const void* A, const void* B, float* C, void* Cb, const float* bias, int M, int N,
-                              int K, int relu, int* err, cudaStream_t st, int stall)
+int gemm_sms()
 {
-    CUtensorMap mapA, mapB;
-    if (!make_map(&mapA, A, M, K, kTm) || !make_map(&mapB, B, N, K, BN)) return cudaErrorInvalidValue;
-    static std::atomic<bool> attr[64];
+    static std::atomic<int> cached{0};
+    int sms = cached.load(std::memory_order_relaxed);
+    if (!sms) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+            sms = 148;
+        cached.store(sms, std::memory_order_relaxed);
+    }
+    return sms;
+}
+
+// Opt-in shared memory of one kernel, once per device.
+template <typename Kernel>
+cudaError_t allow_smem(Kernel* kernel, int bytes, std::atomic<bool> (&done)[64])
+{
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!attr[dev].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmShape<BN>::kSmem);
-        if (e != cudaSuccess) return e;
-        attr[dev].store(true, std::memory_order_release);
-    }
-    const int tiles = (M / kTm) * (N / BN);
-    static std::atomic<int> sms_cached{0};
-    int sms = sms_cached.load(std::memory_order_relaxed);
-    if (!sms) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-        sms_cached.store(sms, std::memory_order_relaxed);
-    }
-    if (!stall && tiles > sms && !getenv("SGB_GEMM_ONE_TILE_PER_CTA")) {
-        // more than one wave: persistent CTAs with two TMEM accumulators
-        static std::atomic<bool> pattr[64];
-        if (!pattr[dev].load(std::memory_order_acquire)) {
-            e = cudaFuncSetAttribute(k_gemm_bf16_pers<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     GemmShape<BN>::kSmem);
+    if (done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done[dev].store(true, std::memory_order_release);
+    return e;
+}
+
+template <int BM, int BN, bool ROWS = false>
+cudaError_t launch_gemm_tiles(const void* A, const void* B, float* C, void* Cb, const float* bias, int M, int N,
+                              int K, int relu, int* err, cudaStream_t st, int stall)
+{
+    using S = GemmShape<BM, BN, ROWS>;
+    CUtensorMap mapA, mapB;
+    const bool mapped = ROWS ? make_map(&mapA, A, K, M, kTk, BM) && make_map(&mapB, B, K, N, kTk, BN)
+                             : make_map(&mapA, A, M, K, BM) && make_map(&mapB, B, N, K, BN);
+    if (!mapped) return cudaErrorInvalidValue;
+    if constexpr (BM == kTm) {
+        const int tiles = (M / BM) * (N / BN), sms = gemm_sms();
+        if (!stall && tiles > sms && !getenv("SGB_GEMM_ONE_TILE_PER_CTA")) {
+            // more than one wave: persistent CTAs with two TMEM accumulators
+            static std::atomic<bool> done[64];
+            const cudaError_t e = allow_smem(k_gemm_bf16_pers<BN>, S::kSmem + kPersStage, done);
             if (e != cudaSuccess) return e;
-            pattr[dev].store(true, std::memory_order_release);
+            k_gemm_bf16_pers<BN><<<sms, kPersThreads, S::kSmem + kPersStage, st>>>(
+                mapA, mapB, C, static_cast<__nv_bfloat16*>(Cb), bias, M, N, K, relu, err);
+            return cudaGetLastError();
         }
-        k_gemm_bf16_pers<BN><<<sms, kPersThreads, GemmShape<BN>::kSmem, st>>>(
-            mapA, mapB, C, static_cast<__nv_bfloat16*>(Cb), bias, M, N, K, relu, err);
-        return cudaGetLastError();
     }
-    const dim3 grid(N / BN, M / kTm);
-    k_gemm_bf16<BN><<<grid, kGemmThreads, GemmShape<BN>::kSmem, st>>>(
+    static std::atomic<bool> done[64];
+    const cudaError_t e = allow_smem(k_gemm_bf16<BM, BN, ROWS>, S::kSmem, done);
+    if (e != cudaSuccess) return e;
+    k_gemm_bf16<BM, BN, ROWS><<<dim3(N / BN, M / BM), kGemmThreads, S::kSmem, st>>>(
         mapA, mapB, C, static_cast<__nv_bfloat16*>(Cb), bias, M, N, K, relu, err, stall);
     return cudaGetLastError();
 }
 }  // namespace
 
-// Tile width: 256 columns when N allows it and the grid still covers the
-// SMs (148 on B200) at least once, 64 when N is not a multiple of 128,
-// else 128.  SGB_GEMM_BN (64, 128, 256) forces a width that divides N.
+// Tiles of 64 rows, 16, 32 or 64 columns, where they fit the SMs in one wave: the
+// narrowest that does.  A product of few tiles is one chain of K steps in each of
+// its CTAs.  A step's loads take what an SM can take in, about 10 KB in 85 ns, so a
+// step of 64 x 16 measured 83 ns, of 64 x 64 107, of 128 x 64 (a stage a step) 227.
+// Else 128 rows and 256 columns when N allows it and the grid still covers the
+// SMs (148 on B200) at least once, 64 when N is not a multiple of 128, else 128.
+// SGB_GEMM_BN (64, 128, 256) forces 128 rows and a width that divides N.
 cudaError_t launch_gemm_bf16(const void* A, const void* B, float* C, void* Cb, const float* bias, int M, int N,
                              int K, int relu, int* err, cudaStream_t st, int stall)
 {
     if (M <= 0 || N <= 0 || K <= 0 || M % kTm || N % 64 || K % kTk) return cudaErrorInvalidValue;
-    int bn = N % 128 ? 64 : (N % 256 == 0 && (long long)(M / kTm) * (N / 256) >= 148) ? 256 : 128;
-    if (const char* force = getenv("SGB_GEMM_BN")) {
+    int bm = kTm, bn = N % 128 ? 64 : (N % 256 == 0 && (long long)(M / kTm) * (N / 256) >= 148) ? 256 : 128;
+    const char* force = getenv("SGB_GEMM_BN");
+    if (force) {
         const int f = atoi(force);
         if ((f == 64 || f == 128 || f == 256) && N % f == 0) bn = f;
+    } else if (!stall) {
+        for (int w = 64; w >= 16; w /= 2)
+            if ((long long)(M / 64) * (N / w) <= gemm_sms()) { bm = 64; bn = w; }
     }
-    switch (bn) {
-    case 256: return launch_gemm_tiles<256>(A, B, C, Cb, bias, M, N, K, relu, err, st, stall);
-    case 128: return launch_gemm_tiles<128>(A, B, C, Cb, bias, M, N, K, relu, err, st, stall);
-    default: return launch_gemm_tiles<64>(A, B, C, Cb, bias, M, N, K, relu, err, st, stall);
-    }
+    auto* launch = bm == 64 ? (bn == 16 ? launch_gemm_tiles<64, 16> : bn == 32 ? launch_gemm_tiles<64, 32>
+                                                                              : launch_gemm_tiles<64, 64>)
+                 : bn == 256 ? launch_gemm_tiles<kTm, 256> : bn == 128 ? launch_gemm_tiles<kTm, 128>
+                                                                       : launch_gemm_tiles<kTm, 64>;
+    return launch(A, B, C, Cb, bias, M, N, K, relu, err, st, stall);
+}
+
+// C = X^T Y, a layer's weight gradient, straight from the row-major operands: 64 x 16
+// tiles (64 x 32 and 64 x 64 where those of 16 and 32 columns do not fit one wave).
+// Transposed copies for the product above cost as much as reading the operands four
+// more times (0.5 ms of a batch of 1024), and their rows of 2 MB at K = 2^20 took
+// its steps from 83 to 156 ns.  Splitting K over CTAs would shorten the chain
+// further, but moves results: over 65536 steps the accumulator's truncated sums are
+// 1e-3 below the sums of parts.
+cudaError_t launch_gemm_rows(const void* X, const void* Y, float* C, int M, int N, int K, int* err, cudaStream_t st)
+{
+    if (M <= 0 || N <= 0 || K <= 0 || M % 64 || N % 64 || (M % 128 && N % 128) || K % kTk) return cudaErrorInvalidValue;
+    const long long tiles = (long long)(M / 64) * (N / 16);
+    auto* launch = tiles <= gemm_sms() ? launch_gemm_tiles<64, 16, true>
+                 : tiles / 2 <= gemm_sms() ? launch_gemm_tiles<64, 32, true> : launch_gemm_tiles<64, 64, true>;
+    return launch(X, Y, C, nullptr, nullptr, M, N, K, 0, err, st, 0);
 }
 
 }  // namespace sgb
@@ -873,8 +1066,13 @@ int solar_gpu_sg_transpose(const void* in_bf16, int R, int C, void* out_bf16, vo
 {
     if (R <= 0 || C <= 0) return 0;
     if ((C + 31) / 32 > 65535) { sgb::set_last_error("transpose: C < 2^21"); return -1; }
-    sgb::k_sg_transpose<<<dim3((R + 31) / 32, (C + 31) / 32), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)in_bf16, R, C, (__nv_bfloat16*)out_bf16);
+    const dim3 grid((R + sgb::kTrTile - 1) / sgb::kTrTile, (C + sgb::kTrTile - 1) / sgb::kTrTile);
+    const auto* in = (const __nv_bfloat16*)in_bf16;
+    auto* out = (__nv_bfloat16*)out_bf16;
+    if (R % 8 == 0 && C % 8 == 0 && ((uintptr_t)in | (uintptr_t)out) % 16 == 0)
+        sgb::k_sg_transpose<true><<<grid, 256, 0, (cudaStream_t)stream>>>(in, R, C, out);
+    else
+        sgb::k_sg_transpose<false><<<grid, 256, 0, (cudaStream_t)stream>>>(in, R, C, out);
     return sg_status(cudaSuccess);
 }
 
@@ -884,8 +1082,12 @@ int solar_gpu_sg_colsum(const void* in_bf16, int R, int C, float* out, void* str
     const int rpb = std::max(64, (R + 1023) / 1024);
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(float) * (size_t)C, (cudaStream_t)stream);
     if (e != cudaSuccess) return sg_status(e);
-    sgb::k_sg_colsum<<<dim3((C + 127) / 128, (R + rpb - 1) / rpb), 128, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)in_bf16, R, C, rpb, out);
+    const bool vec = C % 8 == 0 && (uintptr_t)in_bf16 % 16 == 0;
+    const int groups = vec ? C / 8 : C;
+    const dim3 grid((groups + sgb::kSumGroups - 1) / sgb::kSumGroups, (R + rpb - 1) / rpb);
+    const auto* in = (const __nv_bfloat16*)in_bf16;
+    if (vec) sgb::k_sg_colsum<true><<<grid, 256, 0, (cudaStream_t)stream>>>(in, R, C, rpb, out);
+    else sgb::k_sg_colsum<false><<<grid, 256, 0, (cudaStream_t)stream>>>(in, R, C, rpb, out);
     return sg_status(cudaSuccess);
 }
 
@@ -927,8 +1129,9 @@ int solar_gpu_sg_im2col(const void* X_bf16, int B, int Hi, int Wi, int Cin, int 
         return -1;
     }
     const long long n = (long long)B * (Hi / 2) * (Wi / 2) * (Kp / 8);
-    sgb::k_sg_im2col<<<sg_blocks(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)X_bf16, B, Hi, Wi, Cin, Kp,
-                                                                     (__nv_bfloat16*)cols_bf16);
+    auto* kernel = n <= sgb::kIndex32 ? sgb::k_sg_im2col<unsigned> : sgb::k_sg_im2col<long long>;
+    kernel<<<sg_blocks(n), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)X_bf16, B, Hi, Wi, Cin, Kp,
+                                                           (__nv_bfloat16*)cols_bf16);
     return sg_status(cudaSuccess);
 }
 
@@ -941,8 +1144,9 @@ int solar_gpu_sg_col2im_relu(const float* dcols, const void* X_bf16, int B, int 
         return -1;
     }
     const long long n = (long long)B * Hi * Wi * (Cin / 8);
-    sgb::k_sg_col2im_relu<<<sg_blocks(n), 256, 0, (cudaStream_t)stream>>>(dcols, (const __nv_bfloat16*)X_bf16, B, Hi,
-                                                                          Wi, Cin, Kp, (__nv_bfloat16*)g_bf16);
+    auto* kernel = n <= sgb::kIndex32 ? sgb::k_sg_col2im_relu<unsigned> : sgb::k_sg_col2im_relu<long long>;
+    kernel<<<sg_blocks(n), 256, 0, (cudaStream_t)stream>>>(dcols, (const __nv_bfloat16*)X_bf16, B, Hi, Wi, Cin, Kp,
+                                                           (__nv_bfloat16*)g_bf16);
     return sg_status(cudaSuccess);
 }
 
@@ -978,17 +1182,15 @@ int solar_gpu_sg_transpose_f32(const float* in, int R, int C, float* out, void* 
 }
 
 namespace {
-int gemm_call(const void* A, const void* B, float* C, void* C_bf16, const float* bias, int M, int N, int K, int relu,
-              cudaStream_t st, int stall)
+// Runs launch(error flag) and waits for it.
+extern "C++" {
+template <typename Launch>
+int gemm_call(cudaStream_t st, Launch launch)
 {
-    if (!A || !B || (!C && !C_bf16) || ((uintptr_t)A | (uintptr_t)B | (uintptr_t)C | (uintptr_t)C_bf16) % 16) {
-        sgb::set_last_error("gemm: null or misaligned (16-byte) pointers");
-        return -1;
-    }
     int* err = nullptr;
     cudaError_t e = cudaMallocAsync(&err, sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = sgb::launch_gemm_bf16(A, B, C, C_bf16, bias, M, N, K, relu, err, st, stall);
+    if (e == cudaSuccess) e = launch(err);
     int flag = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, err, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1003,12 +1205,32 @@ int gemm_call(const void* A, const void* B, float* C, void* C_bf16, const float*
     }
     return 0;
 }
+}
+
+int gemm_pointers(const void* A, const void* B, const void* C, const void* C_bf16)
+{
+    if (A && B && (C || C_bf16) && ((uintptr_t)A | (uintptr_t)B | (uintptr_t)C | (uintptr_t)C_bf16) % 16 == 0) return 0;
+    sgb::set_last_error("gemm: null or misaligned (16-byte) pointers");
+    return -1;
+}
 }  // namespace
 
 int solar_gpu_gemm_bf16(const void* A, const void* B, float* C, void* C_bf16, const float* bias, int M, int N,
                         int K, int relu, void* stream)
 {
-    return gemm_call(A, B, C, C_bf16, bias, M, N, K, relu, (cudaStream_t)stream, 0);
+    if (gemm_pointers(A, B, C, C_bf16)) return -1;
+    cudaStream_t st = (cudaStream_t)stream;
+    return gemm_call(st, [&](int* err) { return sgb::launch_gemm_bf16(A, B, C, C_bf16, bias, M, N, K, relu, err, st); });
+}
+
+int solar_gpu_sg_weight_grad(const void* g_bf16, const void* a_bf16, int rows, int n_out, int n_in, float* dW,
+                             void* stream)
+{
+    if (gemm_pointers(g_bf16, a_bf16, dW, nullptr)) return -1;
+    cudaStream_t st = (cudaStream_t)stream;
+    return gemm_call(st, [&](int* err) {
+        return sgb::launch_gemm_rows(g_bf16, a_bf16, dW, n_out, n_in, rows, err, st);
+    });
 }
 
 int solar_gpu_selftest_bounded_wait(void* stream)
@@ -1027,8 +1249,10 @@ int solar_gpu_selftest_bounded_wait(void* stream)
         return -2;
     }
     char* p = static_cast<char*>(buf);
-    const int rc = gemm_call(p, p + a_bytes, reinterpret_cast<float*>(p + a_bytes + b_bytes), nullptr, nullptr, 128,
-                             64, 64, 0, st, 1);
+    const int rc = gemm_call(st, [&](int* err) {
+        return sgb::launch_gemm_bf16(p, p + a_bytes, reinterpret_cast<float*>(p + a_bytes + b_bytes), nullptr, nullptr,
+                                     128, 64, 64, 0, err, st, 1);
+    });
     cudaFreeAsync(buf, st);
     cudaStreamSynchronize(st);
     return rc;

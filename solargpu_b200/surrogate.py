@@ -20,9 +20,10 @@ learn the reflected share (soft binary cross-entropy targets; the prediction
 is the mean of their sigmoids, which gives the one scalar the weight of 16
 bins in the loss); ReLU between layers.  Every
 product, forward and backward, runs on the tensor cores through
-`solar_gpu_gemm_bf16` (bf16 operands, f32 accumulation in TMEM); a
-convolution is im2col + GEMM, its input gradient GEMM + col2im (fused with
-the ReLU mask below it).  Images, labels, the loss, transposes, bias sums
+`solar_gpu_gemm_bf16` (bf16 operands, f32 accumulation in TMEM), the weight
+gradients through `solar_gpu_sg_weight_grad` (the same product over the rows
+of both operands); a convolution is im2col + GEMM, its input gradient GEMM +
+col2im (fused with the ReLU mask below it).  Images, labels, the loss, transposes, bias sums
 and Adam are small CUDA kernels of the library.  Master weights and Adam
 moments are FP32, the GEMMs read bf16 copies.
 
@@ -68,6 +69,7 @@ def _lib():
         L.solar_gpu_sg_hcat.argtypes = [vp, i, vp, i, i, vp, vp]
         L.solar_gpu_sg_relu_grad_cols.argtypes = [vp, i, vp, i, i, i, vp, vp]
         L.solar_gpu_sg_transpose_f32.argtypes = [vp, i, i, vp, vp]
+        L.solar_gpu_sg_weight_grad.argtypes = [vp, vp, i, i, i, vp, vp]
         L.solar_gpu_trace_shadow_subset.argtypes = [vp, C.POINTER(api.SceneDesc), vp, i, vp, C.POINTER(i), vp]
         L._sg_bound = True
     return L
@@ -82,14 +84,6 @@ def _t(torch, x):
     R, Cc = x.shape
     out = torch.empty(Cc, R, dtype=torch.bfloat16, device=x.device)
     api._check(_lib().solar_gpu_sg_transpose(_p(x), R, Cc, _p(out), None))
-    return out
-
-
-def _t32(torch, x):
-    """Transpose of a 2-D f32 CUDA tensor through the library kernel."""
-    R, Cc = x.shape
-    out = torch.empty(Cc, R, dtype=torch.float32, device=x.device)
-    api._check(_lib().solar_gpu_sg_transpose_f32(_p(x), R, Cc, _p(out), None))
     return out
 
 
@@ -234,10 +228,8 @@ class Surrogate:
         for l in range(len(self.W) - 1, -1, -1):
             a = ins[l]
             rows, n_out = g.shape
-            if l < nc:
-                dW[l] = _t32(torch, api.gemm_bf16(_t(torch, a), _t(torch, g)))   # ([K, rows] [rows, N])^T
-            else:
-                dW[l] = api.gemm_bf16(_t(torch, g), _t(torch, a))                # [N, K] = g^T a
+            dW[l] = torch.empty(n_out, a.shape[1], dtype=torch.float32, device=self.dev)
+            api._check(L.solar_gpu_sg_weight_grad(_p(g), _p(a), rows, n_out, a.shape[1], _p(dW[l]), None))   # g^T a
             db[l] = torch.empty(n_out, dtype=torch.float32, device=self.dev)
             api._check(L.solar_gpu_sg_colsum(_p(g), rows, n_out, _p(db[l]), None))
             if l == 0:
