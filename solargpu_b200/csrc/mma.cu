@@ -7,11 +7,24 @@
 // the dense product faster than CUDA cores run the sparse one, and every
 // slab row staged for the group feeds 128 voxels at once.
 //
+// That holds for the cells that many voxels of the group see.  On the 256^2
+// city 71% of a union's cells are seen by at most 8 of the 128 voxels and hold
+// 20% of the weights.  A dense row costs its share of a chunk's 1024 cycles, 16 and more,
+// a weight 2 of an SM's FP32 lanes.  So these light cells stay out of the union:
+//   light    every light weight goes to its cell's list; a warp keeps 16 weights
+//            and their sums in registers, streams the cell's row through (each
+//            8-hour piece is converted once for all 16) and multiplies hour by
+//            hour on packed FP32 pairs, over all blocks of the slab (k_light).
+//            The weights stay in FP32; every sum has a place of its own, and a
+//            voxel's are added in a fixed order (k_mma_accumulate).
+// At most 2 entries a light cell: 1024^2 run 119 ms, 4: 108, 6: 103.9, 8: 103.2, 10:
+// 103.6, 13: 109 (144 without light cells).
+//
 // Once per run (hour-independent):
 //   union    each aligned group of 128 visiting positions: its distinct cells
-//            (shared-memory hash set), sorted descending, written over the
-//            start of the group's weighted-list cells; every weighted entry
-//            gets its slot (index in the union);
+//            (shared-memory hash set, with the entries of each), the light
+//            ones left out, sorted descending; every weighted entry gets its
+//            slot (index in the union);
 //   layout   the union is cut into chunks of 64 rows (the MMA K per stage);
 //            per chunk, its entries are stored as (byte offset in the
 //            shared-memory W tile, fp16 hi, fp16 lo): the weights of voxel t
@@ -28,9 +41,9 @@
 //                        stages, the copies of 3 chunks in flight -- then
 //                        fence the async proxy and arrive on the stage's
 //                        full barrier;
-//   builders (2 x 3 warps) zero one of 3 W stages (K-major, 128-byte swizzle,
+//   builders (3 x 3 warps) zero one of 3 W stages (K-major, 128-byte swizzle,
 //                        A operand, M = voxels) and scatter the chunk's
-//                        entries, fence, arrive; two teams, chunks in turn;
+//                        entries, fence, arrive; three teams, chunks in turn;
 //   MMA (1 thread)       tcgen05.mma kind::f16 M128 N256 K16, 4 per chunk
 //                        and tile (hi, lo), into one of two TMEM accumulators
 //                        (2 x 256 columns), tcgen05.commit frees the stage;
@@ -41,13 +54,14 @@
 //                        accumulator.
 // k_mma_accumulate then adds up each voxel's hour blocks (FP64, Kahan or plain).
 //
-// Bound: the MMAs.  A chunk's eight take 1024 cycles of the tensor pipe (measured
-// alone, B MN-major or K-major alike); here a chunk takes 1630 to 1800, where it
-// took 2300 to 2500 with one launch an hour block, one builder team, the own
-// terms in the epilogue and each chunk published after the wait for the stage of
-// the chunk two ahead.  Reflection of the 1024^2 city 78.5 -> 58.6 ms (1350
-// TFLOP/s of executed fp16 MMA work, the power limit in sight), 512^2 20.1 ->
-// 13.0, 160^2 2.38 -> 1.13, 64^2 1.09 -> 0.13.
+// Bound: the MMAs, and FP32 issue in k_light.  A chunk's eight MMAs take 1024 cycles
+// of the tensor pipe (measured alone, B MN-major or K-major alike); here a chunk takes
+// about 1800, where it took 2300 to 2500 with one launch an hour block, one
+// builder team, the own terms in the epilogue and each chunk published after the
+// wait for the stage of the chunk two ahead.  Without the light cells a chunk has 2.5
+// times the entries: three builder teams take 21.1 ms at 1024^2 where two took 22.9.
+// Reflection of the 1024^2 city 78.5 ms at first, 58.6 with all cells in the
+// unions, 30.8 with light cells; 512^2 20.1, 13.0 and 7.3; 160^2 2.38, 1.13 and 0.73.
 //
 // fp16 I values (RN, unbiased) and split fp16 weights keep the annual error
 // far below 1e-4 (the rounding errors of I are independent across hours).
@@ -56,6 +70,7 @@
 // and frees TMEM before it exits.
 #include "solar_pair.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 
@@ -76,6 +91,11 @@ constexpr int kSmallCap = 8192;             // first pass: unions up to this man
 constexpr int kBuildThreads = 1024;
 constexpr int kLayoutThreads = 512;
 constexpr int kMaxChunks = kUnionCap / kChunk;
+constexpr int kLight = 8;                   // entries of a light cell of a group at most
+constexpr int kLightShift = 3;              // a union takes at most an entry in kLight + 1, so one in 8
+static_assert((1 << kLightShift) <= kLight + 1, "room of a union");
+constexpr unsigned short kLightSlot = 0xFFFF;
+constexpr int kNoSlot = -1;
 constexpr unsigned long long kWaitNs = 1000000000ull;   // 1 s
 constexpr int kMaxDevices = 64;
 
@@ -83,10 +103,11 @@ constexpr int kMaxDevices = 64;
 constexpr int kProducerWarps = 4;           // warps 0-3
 constexpr int kEpilogueWarp0 = 4;           // warps 4-7 (TMEM lane quarters 0-3)
 constexpr int kMmaWarp = 8;
-constexpr int kBuilderWarp0 = 9;            // warps 9-11 and 12-14: two teams, chunks in turn
+constexpr int kBuilderWarp0 = 9;            // warps 9-11, 12-14 and 15-17: three teams, chunks in turn
 constexpr int kBuilderWarps = 3;
-constexpr int kTeams = 2;
-constexpr int kThreads = 15 * 32;
+constexpr int kTeams = 3;
+static_assert(kTeams <= kAStages, "a team that is a stage's second next user would mistake its phase");
+constexpr int kThreads = (kBuilderWarp0 + kTeams * kBuilderWarps) * 32;
 
 // shared memory: 3 x (W hi tile | W lo tile), 4 x slab rows (the hour table
 // is read through L1: every epilogue lane reads the same entry)
@@ -122,23 +143,29 @@ __device__ __forceinline__ void block_sort_desc(uint32_t* keys, int n2)
     }
 }
 
-// The union of group q, in one CTA: cells[e] (0-based cell of weighted entry
-// e) are replaced, from woff[p0] on, by the group's union (descending);
-// slots[e] = index of the entry's cell in it.  Returns false, writing
-// nothing, when the union has more than CAP cells.
-template <int CAP>
-__device__ bool union_group(int q, int N, const long long* __restrict__ woff, int* __restrict__ cells,
+// The union of group q, in one CTA: the distinct cells of its weighted entries
+// (cells[e], 0-based), descending, from ucells[woff[p0]] on (ucells = cells:
+// they are written over the entries' cells); slots[e] = index of the entry's
+// cell in it.  LIGHT: cells with at most kLight entries stay out of the union,
+// which starts at ucells[woff[p0] >> kLightShift]; their entries get the slot
+// kLightSlot and are counted per cell in light.  Returns false, writing
+// nothing, when the group has more than CAP distinct cells.
+template <int CAP, bool LIGHT>
+__device__ bool union_group(int q, int N, const long long* __restrict__ woff, const int* cells, int* ucells,
                             unsigned short* __restrict__ slots, int* __restrict__ unions, int* __restrict__ nch,
-                            uint32_t* sm, int* s_count)
+                            int* __restrict__ light, uint32_t* sm, int* s_count)
 {
     constexpr int kSlots = 2 * CAP;
     constexpr int kBits = CAP == 16384 ? 15 : CAP == 8192 ? 14 : 0;
     static_assert(kBits > 0, "union cap of 8192 or 16384 cells");
     uint32_t* table = sm;                 // [kSlots], key = cell + 1, 0 = empty
     uint32_t* uni = sm + kSlots;          // [CAP]
+    uint32_t* many = uni + CAP;           // LIGHT: [kSlots] bytes, entries of the cell, up to kLight + 1
     const int p0 = q * kGroup, p1 = min(N, p0 + kGroup);
     const long long e0 = woff[p0], e1 = woff[p1];
     for (int i = threadIdx.x; i < kSlots; i += blockDim.x) table[i] = 0u;
+    if (LIGHT)
+        for (int i = threadIdx.x; i < kSlots / 4; i += blockDim.x) many[i] = 0u;
     if (threadIdx.x == 0) *s_count = 0;
     __syncthreads();
     for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
@@ -148,16 +175,42 @@ __device__ bool union_group(int q, int N, const long long* __restrict__ woff, in
             const uint32_t prev = atomicCAS(&table[h], 0u, key);
             if (prev == 0u) {
                 const int at = atomicAdd(s_count, 1);
-                if (at < CAP) uni[at] = key;
+                if (!LIGHT && at < CAP) uni[at] = key;
+            }
+            if (prev == 0u || prev == key) {
+                if (LIGHT) {   // saturating: a caller's list may name a cell any number of times
+                    const int sh = 8 * (int)(h & 3u);
+                    uint32_t old = *reinterpret_cast<volatile uint32_t*>(many + (h >> 2));
+                    while (((old >> sh) & 0xFFu) <= (uint32_t)kLight) {
+                        const uint32_t was = atomicCAS(many + (h >> 2), old, old + (1u << sh));
+                        if (was == old) break;
+                        old = was;
+                    }
+                }
                 break;
             }
-            if (prev == key) break;
             h = (h + 1u) & (kSlots - 1);
         }
     }
     __syncthreads();
-    const int u = *s_count;
+    int u = *s_count;
     if (u > CAP) return false;   // uniform: every thread read the same count
+    const auto is_light = [&](uint32_t h) { return ((many[h >> 2] >> (8 * (h & 3u))) & 0xFFu) <= (uint32_t)kLight; };
+    if (LIGHT) {   // the cells that stay in the union
+        __syncthreads();
+        if (threadIdx.x == 0) *s_count = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < kSlots; i += blockDim.x) {
+            const bool in = table[i] != 0u && !is_light((uint32_t)i);
+            const unsigned bal = __ballot_sync(0xFFFFFFFFu, in);
+            int at = 0;
+            if ((threadIdx.x & 31) == 0 && bal) at = atomicAdd(s_count, __popc(bal));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (in) uni[at + __popc(bal & ((1u << (threadIdx.x & 31)) - 1u))] = table[i];
+        }
+        __syncthreads();
+        u = *s_count;
+    }
     int u2 = 64;
     while (u2 < u) u2 <<= 1;
     for (int i = u + threadIdx.x; i < u2; i += blockDim.x) uni[i] = 0u;
@@ -168,6 +221,16 @@ __device__ bool union_group(int q, int N, const long long* __restrict__ woff, in
     __syncthreads();
     for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
         const int cell = cells[e];
+        if (LIGHT) {
+            const uint32_t key = (uint32_t)cell + 1u;
+            uint32_t h = (key * 2654435761u) >> (32 - kBits);
+            while (table[h] != key) h = (h + 1u) & (kSlots - 1);   // every entry's key is in the table
+            if (is_light(h)) {
+                slots[e] = kLightSlot;
+                atomicAdd(light + cell, 1);
+                continue;
+            }
+        }
         int lo = 0, hi = u - 1;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;
@@ -176,7 +239,8 @@ __device__ bool union_group(int q, int N, const long long* __restrict__ woff, in
         slots[e] = (unsigned short)lo;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < u; i += blockDim.x) cells[e0 + i] = ucell[i];
+    int* dst = ucells + (LIGHT ? e0 >> kLightShift : e0);
+    for (int i = threadIdx.x; i < u; i += blockDim.x) dst[i] = ucell[i];
     if (threadIdx.x == 0) {
         unions[q] = u;
         nch[q] = (u + kChunk - 1) / kChunk;
@@ -187,32 +251,36 @@ __device__ bool union_group(int q, int N, const long long* __restrict__ woff, in
 // First pass, one CTA per group with room for kSmallCap cells (96 KB of
 // shared memory: two CTAs a SM); a group with a larger union is listed in
 // retry[1 ..] (count in retry[0]) and left untouched.
+template <bool LIGHT>
 __global__ void __launch_bounds__(kBuildThreads)
-k_mma_union_small(int N, const long long* __restrict__ woff, int* __restrict__ cells,
+k_mma_union_small(int N, const long long* __restrict__ woff, const int* cells, int* ucells,
                   unsigned short* __restrict__ slots, int* __restrict__ unions, int* __restrict__ nch,
-                  int* __restrict__ retry, int hand_on_all)
+                  int* __restrict__ light, int* __restrict__ retry, int hand_on_all)
 {
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ int s_count;
     const int q = blockIdx.x;
-    if ((hand_on_all || !union_group<kSmallCap>(q, N, woff, cells, slots, unions, nch, sm, &s_count)) &&
+    if ((hand_on_all ||
+         !union_group<kSmallCap, LIGHT>(q, N, woff, cells, ucells, slots, unions, nch, light, sm, &s_count)) &&
         threadIdx.x == 0)
         retry[1 + atomicAdd(retry, 1)] = q;
 }
 
 // Second pass over the listed groups with room for kUnionCap cells; a union
 // above that leaves the group untouched and counts it in *over.
+template <bool LIGHT>
 __global__ void __launch_bounds__(kBuildThreads)
-k_mma_union_large(int N, const long long* __restrict__ woff, int* __restrict__ cells,
+k_mma_union_large(int N, const long long* __restrict__ woff, const int* cells, int* ucells,
                   unsigned short* __restrict__ slots, int* __restrict__ unions, int* __restrict__ nch,
-                  const int* __restrict__ retry, int* __restrict__ over)
+                  int* __restrict__ light, const int* __restrict__ retry, int* __restrict__ over)
 {
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ int s_count;
     const int n = retry[0];
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const int q = retry[1 + i];
-        if (!union_group<kUnionCap>(q, N, woff, cells, slots, unions, nch, sm, &s_count) && threadIdx.x == 0) {
+        if (!union_group<kUnionCap, LIGHT>(q, N, woff, cells, ucells, slots, unions, nch, light, sm, &s_count) &&
+            threadIdx.x == 0) {
             atomicAdd(over, 1);
             unions[q] = 0;
             nch[q] = 0;
@@ -233,12 +301,12 @@ __device__ __forceinline__ unsigned a_offset(int t, int k)
 // One CTA per group.  PASS 0: entries per chunk (ccnt at cbase[q]) and the
 // per-position scale 2^e; PASS 1: the entries at coff (ent must not be
 // read before).  Groups that overflowed the union cap have no chunks.
-template <int PASS>
+template <int PASS, bool LIGHT>
 __global__ void __launch_bounds__(kLayoutThreads)
 k_mma_layout(int N, const long long* __restrict__ woff, const unsigned short* __restrict__ slots,
              const float* __restrict__ wts, const int* __restrict__ nch, const long long* __restrict__ cbase,
              int* __restrict__ ccnt, const long long* __restrict__ coff, uint2* __restrict__ ent,
-             float* __restrict__ scale)
+             float* __restrict__ scale, LightLists ll)
 {
     __shared__ int s_cnt[kMaxChunks];
     __shared__ int s_exp[kGroup];
@@ -263,14 +331,30 @@ k_mma_layout(int N, const long long* __restrict__ woff, const unsigned short* __
         }
     }
     __syncthreads();
-    if (nc == 0) return;
+    if (nc == 0 && !LIGHT) return;
     const long long cb = cbase[q];
     // voxel t owns entries [woff[p0 + t], woff[p0 + t + 1])
     for (int t = warp; t < p1 - p0; t += kLayoutThreads / 32) {
         const int p = p0 + t;
         const float sc = ldexpf(1.0f, -s_exp[t]);
-        for (long long e = woff[p] + lane; e < woff[p + 1]; e += 32) {
-            const int sl = slots[e];
+        int nl = 0;   // light entries of the voxel so far
+        const long long eb = woff[p], ee = woff[p + 1];
+        for (long long e0 = eb; e0 < ee; e0 += 32) {
+            const long long e = e0 + lane;
+            const int sl = e < ee ? slots[e] : kNoSlot;
+            if (LIGHT) {
+                const bool is = sl == kLightSlot;
+                const unsigned bal = __ballot_sync(0xFFFFFFFFu, is);
+                if (PASS == 1 && is) {   // to its cell's list, in any order: each product stands for itself
+                    const int cell = ll.cells[e];
+                    const long long at = ll.off[cell] + (atomicSub(ll.cnt + cell, 1) - 1);
+                    ll.ent[at] = make_uint2((uint32_t)(eb + nl + __popc(bal & ((1u << lane) - 1u))),
+                                            __float_as_uint(wts[e]));
+                }
+                nl += __popc(bal);
+                if (is) continue;
+            }
+            if (sl == kNoSlot) continue;
             const int c = sl / kChunk;
             const int at = atomicAdd(&s_cnt[c], 1);
             if (PASS == 1) {
@@ -281,6 +365,7 @@ k_mma_layout(int N, const long long* __restrict__ woff, const unsigned short* __
                 ent[coff[cb + c] + at] = make_uint2(a_offset(t, sl - c * kChunk), *reinterpret_cast<const unsigned*>(&hl));
             }
         }
+        if (LIGHT && PASS == 1 && lane == 0) ll.many[p] = nl;
     }
     if (PASS == 0) {
         __syncthreads();
@@ -326,6 +411,125 @@ k_solar_slab16(const float4* __restrict__ geo_n, int T, const uint32_t* __restri
         const __half2 h0 = __float22half2_rn(i0), h1 = __float22half2_rn(i1);
         dst[(size_t)g * (kHours / 4)] =
             make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
+    }
+}
+
+// ---- light cells ------------------------------------------------------------------
+
+// One block of the cell's row (8 hours a lane) times the weights of E entries.
+template <int E>
+__device__ __forceinline__ void light_row(const uint4& r, const f32x2 (&w)[E / 2], f32x2 (&acc)[E / 2])
+{
+    const unsigned x[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&x[i]));
+        const f32x2 a = pack2(h.x, h.x), b = pack2(h.y, h.y);
+#pragma unroll
+        for (int j = 0; j < E / 2; ++j) acc[j] = fma2(w[j], a, acc[j]);
+#pragma unroll
+        for (int j = 0; j < E / 2; ++j) acc[j] = fma2(w[j], b, acc[j]);
+    }
+}
+
+// n (at most E) entries of one cell over nb hour blocks; row: this lane's piece
+// of the cell's row in the first block, `stride` pieces to the next one's.
+template <int E>
+__device__ __forceinline__ void light_cell(const uint4* __restrict__ row, size_t stride, int nb,
+                                           const uint2* __restrict__ ent, int n, float* __restrict__ val, int lane)
+{
+    constexpr int kAhead = 2;   // rows in flight (4: +6%, 6: +14%, for the registers they take)
+    const uint2 en = lane < n ? __ldg(ent + lane) : make_uint2(0u, 0u);
+    uint4 r[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) r[i] = i < nb ? __ldg(row + i * stride) : make_uint4(0u, 0u, 0u, 0u);
+    f32x2 w[E / 2], acc[E / 2];
+#pragma unroll
+    for (int j = 0; j < E / 2; ++j) {
+        w[j] = pack2(__uint_as_float(__shfl_sync(0xFFFFFFFFu, en.y, 2 * j)),
+                     __uint_as_float(__shfl_sync(0xFFFFFFFFu, en.y, 2 * j + 1)));
+        acc[j] = 0ull;
+    }
+    for (int b = 0; b < nb; b += kAhead) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            if (b + i >= nb) break;
+            const uint4 x = r[i];
+            if (b + i + kAhead < nb) r[i] = __ldg(row + (size_t)(b + i + kAhead) * stride);
+            light_row<E>(x, w, acc);
+        }
+    }
+    // the lanes' sums of every entry: lane l ends with entry l / (32 / E)
+    float a[E];
+#pragma unroll
+    for (int j = 0; j < E / 2; ++j) {
+        const float2 v = unpack2(acc[j]);
+        a[2 * j] = v.x;
+        a[2 * j + 1] = v.y;
+    }
+#pragma unroll
+    for (int k = E / 2, o = 16; o > 0; k >>= 1, o >>= 1) {
+        if (k >= 1) {
+#pragma unroll
+            for (int j = 0; j < k; ++j) {
+                const float keep = (lane & o) ? a[j + k] : a[j], give = (lane & o) ? a[j] : a[j + k];
+                a[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, o);
+            }
+        } else {
+            a[0] += __shfl_xor_sync(0xFFFFFFFFu, a[0], o);
+        }
+    }
+    const int i = lane / (32 / E);
+    const uint32_t at = __shfl_sync(0xFFFFFFFFu, en.x, i);
+    if (lane % (32 / E) == 0 && i < n) val[at] = a[0];
+}
+
+constexpr int kLightWarps = 8;
+constexpr int kLightWindow = 128;   // entries of a warp (64: +2% in a run, 32: +20%)
+
+// Products of the light entries with the rows of their cells, hour by hour,
+// summed over the nb hour blocks of the slab: val[entry].
+__global__ void __launch_bounds__(kLightWarps * 32, 4)
+k_light(const uint4* __restrict__ slab, int T, int nb, int window, const long long* __restrict__ off,
+        const uint2* __restrict__ ent, float* __restrict__ val)
+{
+    const int lane = threadIdx.x & 31;
+    const long long total = __ldg(off + T);
+    long long at = ((long long)blockIdx.x * kLightWarps + (threadIdx.x >> 5)) * window;
+    const long long end = min(total, at + window);
+    if (at >= end) return;
+    int lo = 0, hi = T - 1;   // the last cell that starts at or before the first entry
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(off + mid) <= at) lo = mid; else hi = mid - 1;
+    }
+    int cell = lo;
+    const size_t stride = (size_t)T * (kHours / 8);
+    while (at < end) {
+        // the cell of entry `at`: the first one that ends after it
+        long long stop = 0;
+        for (;;) {
+            const int c = cell + lane;
+            const long long e = c < T ? __ldg(off + c + 1) : total;
+            const unsigned past = __ballot_sync(0xFFFFFFFFu, e > at);
+            if (past) {
+                const int i = __ffs(past) - 1;
+                cell += i;
+                stop = __shfl_sync(0xFFFFFFFFu, e, i);
+                break;
+            }
+            cell += 32;
+        }
+        int n = (int)(min(stop, end) - at);
+        const uint4* row = slab + (size_t)cell * (kHours / 8) + lane;
+        while (n > 0) {
+            int k;
+            if (n > 8) light_cell<16>(row, stride, nb, ent + at, k = min(n, 16), val, lane);
+            else if (n > 4) light_cell<8>(row, stride, nb, ent + at, k = n, val, lane);
+            else light_cell<4>(row, stride, nb, ent + at, k = n, val, lane);
+            at += k;
+            n -= k;
+        }
     }
 }
 
@@ -411,7 +615,8 @@ __device__ __forceinline__ void mma_commit(unsigned bar)
 // fill the GPU with several hour blocks at once.
 struct MmaTiles {
     int N, T, NG, items, rot;  // item n: hour block n / NG, group (n + rot * (n / NG)) % NG
-    const long long* woff;     // [N + 1]; the union of group q starts at woff[128 q]
+    const long long* woff;     // [N + 1]; the union of group q starts at woff[128 q] >> shift
+    int shift;
     const int* cells;          // union cells (descending) per group
     const int* unions;         // [NG] union size
     const long long* cbase;    // [NG + 1] first chunk of each group
@@ -444,7 +649,7 @@ struct Cursor {
             if (c * kChunk < u) break;
         }
         if (n < mt.items) {
-            ub = __ldg(mt.woff + (long long)q * kGroup);
+            ub = __ldg(mt.woff + (long long)q * kGroup) >> mt.shift;
             cb = __ldg(mt.cbase + q);
             row0 = (long long)mt.block_of(n) * mt.T;
         }
@@ -619,16 +824,16 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, float* __restrict__ 
         }
         __syncwarp();
     } else if (warp >= kBuilderWarp0) {
-        // ---- builders: zero the W tiles, scatter the chunk's weights.  Two teams
+        // ---- builders: zero the W tiles, scatter the chunk's weights.  The teams
         // take the chunks in turn, and a team loads the entries of its next chunk
-        // into registers while the other one builds: one team's chunk takes 1300
+        // into registers while the others build: one team's chunk takes 1300
         // cycles and more, the chunk's MMAs 1024
         const int team = (warp - kBuilderWarp0) / kBuilderWarps;
         const int bt = threadIdx.x - (kBuilderWarp0 + team * kBuilderWarps) * 32;
         constexpr int kBuilders = kBuilderWarps * 32;
         constexpr int kPref = 16;   // entries a thread holds ahead (8: +11%, 12: +1.6%, 20: +2%); more load at scatter
         Cursor cur(mt, blockIdx.x);
-        if (team && cur.valid(mt)) cur.advance(mt);
+        for (int i = 0; i < team && cur.valid(mt); ++i) cur.advance(mt);
         uint2 pre[kPref];
         long long pe0 = 0, pe1 = 0;
         auto prefetch = [&]() {
@@ -676,8 +881,7 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, float* __restrict__ 
             if (bt == 0) bar_arrive(su32(&aready[s]));
             // the team's next chunk's entries (after the arrive: their latency stays
             // off the MMA's path)
-            cur.advance(mt);
-            if (cur.valid(mt)) cur.advance(mt);
+            for (int i = 0; i < kTeams && cur.valid(mt); ++i) cur.advance(mt);
             prefetch();
             k += kTeams;
         }
@@ -753,8 +957,8 @@ k_reflect_mma(const __half* __restrict__ slab, MmaTiles mt, float* __restrict__ 
 // accumulators are read / kept).
 template <int MODE>
 __global__ void __launch_bounds__(256)
-k_mma_accumulate(const int* __restrict__ order, int N, int nb, const float* __restrict__ sums, Accum acc, bool first,
-                 bool last, float* __restrict__ out)
+k_mma_accumulate(const int* __restrict__ order, int N, int nb, const float* __restrict__ sums, LightLists ll,
+                 const long long* __restrict__ woff, Accum acc, bool first, bool last, float* __restrict__ out)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= N) return;
@@ -766,9 +970,7 @@ k_mma_accumulate(const int* __restrict__ order, int N, int nb, const float* __re
         else a32 = acc.f32[v];
         if (MODE == 1) comp = acc.comp[v];
     }
-#pragma unroll 4
-    for (int hb = 0; hb < nb; ++hb) {
-        const float x = __ldg(sums + (size_t)hb * N + p);
+    const auto add = [&](float x) {
         if (MODE == 0) {
             a64 += (double)x;
         } else if (MODE == 1) {
@@ -779,6 +981,14 @@ k_mma_accumulate(const int* __restrict__ order, int N, int nb, const float* __re
         } else {
             a32 = __fadd_rn(a32, x);
         }
+    };
+#pragma unroll 4
+    for (int hb = 0; hb < nb; ++hb) add(__ldg(sums + (size_t)hb * N + p));
+    if (ll.many) {   // the voxel's light entries, as one more block
+        const float* val = ll.val + woff[p];
+        float x = 0.0f;
+        for (int i = 0, n = __ldg(ll.many + p); i < n; ++i) x += __ldg(val + i);
+        add(x);
     }
     if (last) {
         out[v] = MODE == 0 ? (float)a64 : a32;
@@ -823,39 +1033,59 @@ cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<bool> (&done)[kMaxDev
 
 int mma_group_count(int N) { return (N + kGroup - 1) / kGroup; }
 
-cudaError_t launch_mma_union(int N, const long long* woff, int* cells, unsigned short* slots, int* unions, int* nch,
-                             int* over, int* retry, cudaStream_t st)
+// Light cells from 20,000 voxels on: below, the launches for them and their lists
+// cost more than the MMAs they save (runs of 112^2, 17,500 voxels: 1.94 ms with them,
+// 1.88 without; 128^2, 23,000: 2.26 and 2.36; 64^2 1.14 and 1.07).  Entries are
+// numbered with 32 bits.
+bool mma_light_ok(int N, long long entries) { return N >= 20000 && entries < 0xFFFFFFFFll; }
+long long mma_union_room(long long entries) { return (entries >> kLightShift) + 1; }
+
+cudaError_t launch_mma_union(int N, const long long* woff, int* cells, int* ucells, unsigned short* slots, int* unions,
+                             int* nch, int* light, int* over, int* retry, cudaStream_t st)
 {
     const int NG = mma_group_count(N);
     if (NG <= 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(retry, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    const size_t small = sizeof(uint32_t) * (size_t)(3 * kSmallCap);
-    const size_t large = sizeof(uint32_t) * (size_t)(kHashSlots + kUnionCap);
-    static std::atomic<bool> attr_s[kMaxDevices], attr_l[kMaxDevices];
-    if ((e = allow_smem(k_mma_union_small, small, attr_s)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_mma_union_large, large, attr_l)) != cudaSuccess) return e;
+    // with the light cells' byte a slot: 112 KB (two CTAs a SM) and 224 KB
+    const size_t small = sizeof(uint32_t) * (size_t)(3 * kSmallCap) + (light ? 2 * kSmallCap : 0);
+    const size_t large = sizeof(uint32_t) * (size_t)(kHashSlots + kUnionCap) + (light ? kHashSlots : 0);
+    static std::atomic<bool> attr_s[2][kMaxDevices], attr_l[2][kMaxDevices];
+    const auto ks = light ? k_mma_union_small<true> : k_mma_union_small<false>;
+    const auto kl = light ? k_mma_union_large<true> : k_mma_union_large<false>;
+    if ((e = allow_smem(ks, small, attr_s[light ? 1 : 0])) != cudaSuccess) return e;
+    if ((e = allow_smem(kl, large, attr_l[light ? 1 : 0])) != cudaSuccess) return e;
     // SGB_UNION_SECOND_PASS=1 hands every group to the second pass (tests use
     // it to check that pass; the unions are the same either way)
     const char* env = std::getenv("SGB_UNION_SECOND_PASS");
     const int all = (env && env[0] == '1') ? 1 : 0;
-    k_mma_union_small<<<NG, kBuildThreads, small, st>>>(N, woff, cells, slots, unions, nch, retry, all);
+    ks<<<NG, kBuildThreads, small, st>>>(N, woff, cells, ucells, slots, unions, nch, light, retry, all);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // the groups the first pass listed (usually few; the grid exits at once when none)
-    k_mma_union_large<<<mma_sms(), kBuildThreads, large, st>>>(N, woff, cells, slots, unions, nch, retry, over);
+    kl<<<mma_sms(), kBuildThreads, large, st>>>(N, woff, cells, ucells, slots, unions, nch, light, retry, over);
     return cudaGetLastError();
 }
 
 cudaError_t launch_mma_layout(int pass, int N, const long long* woff, const unsigned short* slots, const float* wts,
                               const int* nch, const long long* cbase, int* ccnt, const long long* coff, uint2* ent,
-                              float* scale, cudaStream_t st)
+                              float* scale, const LightLists& ll, cudaStream_t st)
 {
     const int NG = mma_group_count(N);
     if (NG <= 0) return cudaSuccess;
-    if (pass == 0)
-        k_mma_layout<0><<<NG, kLayoutThreads, 0, st>>>(N, woff, slots, wts, nch, cbase, ccnt, coff, ent, scale);
-    else
-        k_mma_layout<1><<<NG, kLayoutThreads, 0, st>>>(N, woff, slots, wts, nch, cbase, ccnt, coff, ent, scale);
+    const auto k = ll.many ? (pass == 0 ? k_mma_layout<0, true> : k_mma_layout<1, true>)
+                           : (pass == 0 ? k_mma_layout<0, false> : k_mma_layout<1, false>);
+    k<<<NG, kLayoutThreads, 0, st>>>(N, woff, slots, wts, nch, cbase, ccnt, coff, ent, scale, ll);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_light(const void* slab16, int T, int nb, const LightLists& ll, cudaStream_t st)
+{
+    if (!ll.many || ll.total <= 0 || nb <= 0) return cudaSuccess;
+    // entries of a warp: enough to share the rows, fewer where the GPU would not be full
+    const int window = (int)std::max<long long>(16, std::min<long long>(kLightWindow, ll.total / (24 * mma_sms())) & ~15ll);
+    const long long warps = (ll.total + window - 1) / window;
+    k_light<<<(unsigned)((warps + kLightWarps - 1) / kLightWarps), kLightWarps * 32, 0, st>>>(
+        static_cast<const uint4*>(slab16), T, nb, window, ll.off, ll.ent, ll.val);
     return cudaGetLastError();
 }
 
@@ -886,20 +1116,21 @@ cudaError_t launch_reflect_mma(const void* slab16, int T, const MmaLists& ml, in
     if ((long long)NG * nb > 0x7FFFFFFFLL - 4096) return cudaErrorInvalidValue;
     const int items = NG * nb, grid = items < mma_sms() ? items : mma_sms();
     // with a multiple of the grid's size a CTA would meet the same groups in every hour block
-    MmaTiles mt{ml.N, T, NG, items, NG % grid == 0 ? 1 : 0, ml.woff, ml.cells, ml.unions, ml.cbase, ml.coff,
+    MmaTiles mt{ml.N, T, NG, items, NG % grid == 0 ? 1 : 0, ml.woff, ml.light.many ? kLightShift : 0, ml.cells, ml.unions, ml.cbase, ml.coff,
                 reinterpret_cast<const uint2*>(ml.ent), ml.scale};
     k_reflect_mma<<<grid, kThreads, kSmemBytes, st>>>(static_cast<const __half*>(slab16), mt, sums, err);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mma_accumulate(const int* order, int N, int nb, const float* sums, const Accum& acc, bool first,
-                                  bool last, float* out, cudaStream_t st)
+cudaError_t launch_mma_accumulate(const int* order, int nb, const float* sums, const MmaLists& ml, const Accum& acc,
+                                  bool first, bool last, float* out, cudaStream_t st)
 {
+    const int N = ml.N;
     if (N <= 0) return cudaSuccess;
     const unsigned grid = (unsigned)((N + 255) / 256);
-    if (acc.mode == 0) k_mma_accumulate<0><<<grid, 256, 0, st>>>(order, N, nb, sums, acc, first, last, out);
-    else if (acc.mode == 1) k_mma_accumulate<1><<<grid, 256, 0, st>>>(order, N, nb, sums, acc, first, last, out);
-    else k_mma_accumulate<2><<<grid, 256, 0, st>>>(order, N, nb, sums, acc, first, last, out);
+    if (acc.mode == 0) k_mma_accumulate<0><<<grid, 256, 0, st>>>(order, N, nb, sums, ml.light, ml.woff, acc, first, last, out);
+    else if (acc.mode == 1) k_mma_accumulate<1><<<grid, 256, 0, st>>>(order, N, nb, sums, ml.light, ml.woff, acc, first, last, out);
+    else k_mma_accumulate<2><<<grid, 256, 0, st>>>(order, N, nb, sums, ml.light, ml.woff, acc, first, last, out);
     return cudaGetLastError();
 }
 

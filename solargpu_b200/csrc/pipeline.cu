@@ -115,7 +115,7 @@ struct solar_gpu_context {
         grp_cell, grp_w, w_cnt, w_off, w_tmp, w_cell, w_val, order_first, order_inv, tile_flag, tile_pos,
         tile_start, tile_union, tile_slot, tile_rows, tile_gcnt, tile_gnch, tile_gbase, tile_tbase, tile_table,
         tile_erow, tile_ew, chunk_perm, chunk_flag, chunk_pos, chunk_tmp, mma_union, mma_nch, mma_cbase,
-        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, hour_sums, mma_retry, cone, cone_tmp, cone_specs,
+        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, mma_ucell, light_many, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, hour_sums, mma_retry, cone, cone_tmp, cone_specs,
         sweep_blocks, sweep_line, box;
     int* h_scalars = nullptr;   // pinned host scratch for small read-backs
     long long mem_limit = 0;    // device bytes the buffers may hold (0: no limit)
@@ -151,7 +151,7 @@ struct solar_gpu_context {
     cudaStream_t kt_stream = nullptr;
 };
 
-static constexpr int kNumBufs = 87;
+static constexpr int kNumBufs = 89;
 extern "C" {
 static void all_bufs(solar_gpu_context* c, DevBuf** out);   // defined with the exports below
 }
@@ -652,13 +652,14 @@ cudaError_t enqueue_hours(solar_gpu_context* c, const HourLoop& h, cudaStream_t 
             }
             if (le == cudaSuccess) {
                 KScope k(c, SOLAR_GPU_KT_REFLECT);
-                le = launch_reflect_mma(h.slab16, h.T, h.ml, nb, h.sums, h.err, st);
+                le = launch_light(h.slab16, h.T, nb, h.ml.light, st);
+                if (le == cudaSuccess) le = launch_reflect_mma(h.slab16, h.T, h.ml, nb, h.sums, h.err, st);
             }
             if (le == cudaSuccess) {
                 KScope k(c, SOLAR_GPU_KT_FINALIZE);
-                le = launch_mma_accumulate(h.order, h.N, nb, h.sums, h.acc, j0 == 0, j0 + step >= h.Hd, h.out, st);
+                le = launch_mma_accumulate(h.order, nb, h.sums, h.ml, h.acc, j0 == 0, j0 + step >= h.Hd, h.out, st);
             }
-            c->launches += 4;
+            c->launches += h.ml.light.total > 0 ? 5 : 4;
         }
         // no daylight hour: nothing was accumulated
         if (h.Hd <= 0) le = cudaMemsetAsync(h.out, 0, sizeof(float) * (size_t)h.N, st);
@@ -820,21 +821,39 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
                 RK(ensure(c, c->mma_cbase, sizeof(long long) * ((size_t)NG + 1)));
                 RK(ensure(c, c->mma_over, sizeof(long long)));
                 RK(ensure(c, c->mma_retry, sizeof(int) * ((size_t)NG + 1)));
+                // Light cells take memory of their own (a byte a weight), so not under a
+                // memory limit, and keep the weights' buffer, so not where it is released below.
+                // Their counts and offsets go where the visiting order was built.
+                bool light = c->mem_limit <= 0 && mma_light_ok(N, Ew) &&
+                             c->w_val.cap + c->tile_slot.cap <= c->dev_total / 16;
+                if (light && (ensure(c, c->mma_ucell, sizeof(int) * (size_t)mma_union_room(Ew)) != SOLAR_GPU_OK ||
+                              ensure(c, c->light_many, sizeof(int) * (size_t)N) != SOLAR_GPU_OK)) {
+                    (void)cudaGetLastError();   // no room after all
+                    light = false;
+                }
+                LightLists ll{};
+                int* ucells = light ? as<int>(c->mma_ucell) : as<int>(c->w_cell);
                 {
                     KScope k(c, SOLAR_GPU_KT_GROUP);
                     CK(cudaMemsetAsync(c->mma_over.p, 0, sizeof(long long), st));
-                    CK(launch_mma_union(N, as<long long>(c->w_off), as<int>(c->w_cell),
+                    if (light) CK(cudaMemsetAsync(c->order_cnt.p, 0, sizeof(int) * (size_t)T, st));
+                    CK(launch_mma_union(N, as<long long>(c->w_off), as<int>(c->w_cell), ucells,
                                         as<unsigned short>(c->tile_slot), as<int>(c->mma_union), as<int>(c->mma_nch),
-                                        as<int>(c->mma_over), as<int>(c->mma_retry), st));
+                                        light ? as<int>(c->order_cnt) : nullptr, as<int>(c->mma_over),
+                                        as<int>(c->mma_retry), st));
                     CK(launch_scan_counts(as<int>(c->mma_nch), NG, 0, as<long long>(c->mma_cbase),
                                           as<long long>(c->w_tmp), nullptr, st));
+                    if (light)
+                        CK(launch_scan_counts(as<int>(c->order_cnt), T, 0, as<long long>(c->order_cur),
+                                              as<long long>(c->order_tmp), nullptr, st));
                 }
                 long long over = 0, C = 0;
                 RK(read_ll(c, as<long long>(c->mma_over), &over, st));
                 RK(read_ll(c, as<long long>(c->mma_cbase) + NG, &C, st));
-                c->launches += 4;
+                if (light) RK(read_ll(c, as<long long>(c->order_cur) + T, &ll.total, st));
+                c->launches += light ? 7 : 4;
                 if (over != 0) {
-                    // the union build rewrote the cells of the groups it kept: rebuild the lists
+                    // the union build may have rewritten the cells of the groups it kept: rebuild the lists
                     mma = false;
                     V = 64;
                     KScope k(c, SOLAR_GPU_KT_GROUP);
@@ -846,18 +865,26 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
                     RK(ensure(c, c->mma_coff, sizeof(long long) * ((size_t)C + 1)));
                     RK(ensure(c, c->mma_scale, sizeof(float) * (size_t)N));
                     RK(ensure(c, c->mma_ent, 8 * (size_t)(Ew + 1)));
+                    if (light) {   // after the unions' entries; the weights are dead once these are placed
+                        ll.cells = as<int>(c->w_cell);
+                        ll.cnt = as<int>(c->order_cnt);
+                        ll.off = as<long long>(c->order_cur);
+                        ll.ent = static_cast<uint2*>(c->mma_ent.p) + (Ew - ll.total);
+                        ll.many = as<int>(c->light_many);
+                        ll.val = as<float>(c->w_val);
+                    }
                     {
                         KScope k(c, SOLAR_GPU_KT_GROUP);
                         CK(launch_mma_layout(0, N, as<long long>(c->w_off), as<unsigned short>(c->tile_slot),
                                              as<float>(c->w_val), as<int>(c->mma_nch), as<long long>(c->mma_cbase),
-                                             as<int>(c->mma_ccnt), nullptr, nullptr, as<float>(c->mma_scale), st));
+                                             as<int>(c->mma_ccnt), nullptr, nullptr, as<float>(c->mma_scale), ll, st));
                         RK(ensure(c, c->chunk_tmp, sizeof(long long) * scan_scratch_elems((int)C)));
                         CK(launch_scan_counts(as<int>(c->mma_ccnt), (int)C, 0, as<long long>(c->mma_coff),
                                               as<long long>(c->chunk_tmp), nullptr, st));
                         CK(launch_mma_layout(1, N, as<long long>(c->w_off), as<unsigned short>(c->tile_slot),
                                              as<float>(c->w_val), as<int>(c->mma_nch), as<long long>(c->mma_cbase),
                                              as<int>(c->mma_ccnt), as<long long>(c->mma_coff),
-                                             static_cast<uint2*>(c->mma_ent.p), as<float>(c->mma_scale), st));
+                                             static_cast<uint2*>(c->mma_ent.p), as<float>(c->mma_scale), ll, st));
                     }
                     c->launches += 3;
                     c->group_entries = Ew;
@@ -872,7 +899,8 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
                     }
                     ml.N = N;
                     ml.woff = as<long long>(c->w_off);
-                    ml.cells = as<int>(c->w_cell);
+                    ml.cells = ucells;
+                    ml.light = ll;
                     ml.unions = as<int>(c->mma_union);
                     ml.cbase = as<long long>(c->mma_cbase);
                     ml.coff = as<long long>(c->mma_coff);
@@ -1121,7 +1149,8 @@ int run_device_impl(solar_gpu_context* c, const solar_gpu_options* o, const sola
         CK(cudaStreamSynchronize(st));
         DevBuf* stage23[] = {&c->slab, &c->slab16, &c->hour_sums, &c->w_cnt, &c->w_off, &c->w_cell, &c->w_val, &c->grp_cell,
                              &c->grp_w, &c->tile_slot, &c->tile_erow, &c->tile_ew, &c->tile_table, &c->mma_ent,
-                             &c->mma_ccnt, &c->mma_coff, &c->mma_scale, &c->hourly, &c->csr_ids, &c->barle_bytes};
+                             &c->mma_ccnt, &c->mma_coff, &c->mma_scale, &c->mma_ucell, &c->light_many, &c->hourly, &c->csr_ids,
+                             &c->barle_bytes};
         for (DevBuf* b : stage23) {
             if (b->p) CK(cudaFree(b->p));
             b->p = nullptr;
@@ -1353,6 +1382,7 @@ static void all_bufs(solar_gpu_context* c, DevBuf** out)
                                 &c->tile_table, &c->tile_erow, &c->tile_ew, &c->chunk_perm, &c->chunk_flag,
                                 &c->chunk_pos, &c->chunk_tmp, &c->mma_union, &c->mma_nch, &c->mma_cbase,
                                 &c->mma_ccnt, &c->mma_coff, &c->mma_ent, &c->mma_scale, &c->mma_over, &c->slab16,
+                                &c->mma_ucell, &c->light_many,
                                 &c->dd_ovf, &c->vox_cnt, &c->vox_off, &c->vox_tmp, &c->gpad, &c->hour_sums, &c->mma_retry,
                                 &c->cone, &c->cone_tmp, &c->cone_specs,
                                 &c->sweep_blocks, &c->sweep_line, &c->box};

@@ -254,40 +254,59 @@ cudaError_t launch_reflect_tile(int B, const float* slab, const TileLists& tl, c
 
 // tensor-core reflection (mma.cu): groups of 128 visiting positions, hour
 // blocks of 256, fp16 slab of the top cells.
+//
+// Light cells: those that few voxels of a group see stay out of its union; their
+// entries go to lists by cell (many == nullptr: all cells are in the unions).
+struct LightLists {
+    const int* cells;          // [entries] cells of the weighted lists
+    int* cnt;                  // [T] light entries of each cell (counted down while they are placed)
+    const long long* off;      // [T + 1] scan of cnt
+    uint2* ent;                // [total] by cell: x = index in val, y = weight (float bits)
+    int* many;                 // [N] light entries of each visiting position
+    float* val;                // [entries] position p's from woff[p] on: weight times the cell's hours, summed
+    long long total;
+};
 struct MmaLists {
     int N;
-    const long long* woff;     // [N + 1] weighted-list offsets; the union of group q starts at woff[128 q]
-    const int* cells;          // union cells per group (written over the weighted cells)
+    const long long* woff;     // [N + 1] weighted-list offsets, which also place the unions (mma_union_room)
+    const int* cells;          // union cells per group
     const int* unions;         // [groups] union size
     const long long* cbase;    // [groups + 1] first chunk of each group
     const long long* coff;     // [chunks + 1] first entry of each chunk
     const void* ent;           // [entries] 8 bytes: W-tile byte offset, fp16 hi, fp16 lo
     const float* scale;        // [N] per visiting position: 2^e undoing the weight scaling
+    LightLists light;
 };
 constexpr int kMmaGroup = 128;
 constexpr int kMmaHours = 256;
 constexpr int kMmaChunk = 64;
 int mma_group_count(int N);
-// Union of each group (cells rewritten in place, slots per entry, union size
-// and chunk count per group); *over counts groups above the union cap.
-// retry: groups + 1 ints of scratch (groups the small first pass hands on).
-cudaError_t launch_mma_union(int N, const long long* woff, int* cells, unsigned short* slots, int* unions, int* nch,
-                             int* over, int* retry, cudaStream_t st);
+// Union of each group (slots per entry, union size and chunk count per group);
+// *over counts groups above the union cap.  retry: groups + 1 ints of scratch
+// (groups the small first pass hands on).  light == nullptr: the unions are
+// written over the cells (ucells = cells).  Else light [T] (zero) counts the
+// light entries of each cell, and ucells holds mma_union_room cells.
+bool mma_light_ok(int N, long long entries);
+long long mma_union_room(long long entries);
+cudaError_t launch_mma_union(int N, const long long* woff, int* cells, int* ucells, unsigned short* slots, int* unions,
+                             int* nch, int* light, int* over, int* retry, cudaStream_t st);
 // pass 0: entries per chunk (ccnt at cbase) and the per-position scale;
-// pass 1: the entries at coff (the scan of ccnt).
+// pass 1: the entries at coff (the scan of ccnt), the light ones at ll.off.
 cudaError_t launch_mma_layout(int pass, int N, const long long* woff, const unsigned short* slots, const float* wts,
                               const int* nch, const long long* cbase, int* ccnt, const long long* coff, uint2* ent,
-                              float* scale, cudaStream_t st);
+                              float* scale, const LightLists& ll, cudaStream_t st);
+// ll.val over the slab's nb hour blocks.
+cudaError_t launch_light(const void* slab16, int T, int nb, const LightLists& ll, cudaStream_t st);
 // nb hour blocks from hour j0 on: slab16 [nb][T][256] fp16.
 cudaError_t launch_solar_slab16(const DevGeom& g, int T, const uint32_t* shadow, int words32, const HourEntry* table,
                                 int j0, int nb, void* slab16, cudaStream_t st);
 // sums [nb][N]: adds each hour block's reflected sum, by visiting position.
 cudaError_t launch_reflect_mma(const void* slab16, int T, const MmaLists& ml, int nb, float* sums, int* err,
                                cudaStream_t st);
-// Accumulates nb hour blocks' sums; first / last: the year begins / ends with
-// them (out is written).
-cudaError_t launch_mma_accumulate(const int* order, int N, int nb, const float* sums, const Accum& acc, bool first,
-                                  bool last, float* out, cudaStream_t st);
+// Accumulates nb hour blocks' sums and the light entries' over them; first /
+// last: the year begins / ends with them (out is written).
+cudaError_t launch_mma_accumulate(const int* order, int nb, const float* sums, const MmaLists& ml, const Accum& acc,
+                                  bool first, bool last, float* out, cudaStream_t st);
 
 // voxelization (voxel.cu): wall voxels per cell, then the packed arrays
 // (tops [0, T), walls after them at T + off[cell] + v).
