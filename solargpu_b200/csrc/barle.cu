@@ -7,23 +7,39 @@
 //   length byte per run, then payload (4-bit deltas two per byte, high nibble
 //   first; wider deltas big-endian).
 //
-// One warp per voxel.  The sort (bitonic, shared memory), delta/width
-// classification and run detection (ballot + popc) are warp-parallel; the
-// run optimiser is the reference's sequential fixpoint and runs on one lane
-// over the (short) run list; payload bytes are written lane-parallel.
-// Two passes: k_barle_size computes each stream's byte count (and leaves the
-// sorted list and, room permitting, its optimised runs in the row), a scan
-// turns counts into offsets, k_barle_write packs the bytes.
+// One warp per voxel.  Lists of up to 1024 ids (almost all) are encoded in one
+// pass, in registers (k_barle_encode): a lane holds 8, 16 or 32 consecutive
+// ids, sorted bitonically over lanes by shuffles, and every step after the sort
+// is a short loop over a lane's own ids with one scan over the warp.  That needs
+// the run optimiser without its sequential fixpoint:
+//
+//   A pass merges a run of one id into the run before it when that is one class
+//   wider, going on after the merged one.  So run r is merged if that holds for
+//   (r - 1, r) and r - 1 was not merged itself, a chain of at most four classes.
+//   No later pass finds more: a run that was not merged keeps the run before it
+//   or, if that was merged, meets the one before that, two classes wider or more.
+//   A merged run has one id, so merging means giving the id the next class; the
+//   final runs are the maximal ones of these classes.
+//
+// The stream goes after the sorted list in the voxel's row, a scan turns the
+// sizes into offsets, and k_barle_copy moves the streams there.  Longer lists (up
+// to one id a direction) take two passes with the reference's own loop on one
+// lane: k_barle_size (sizes; sorted list and, room permitting, its runs left in
+// the row) and k_barle_write.
+//
+// Bound: instructions (the sort's shuffles first); the one-lane loops and the
+// run-by-run writes of the two passes were latency.  Sizes, offsets and streams:
+// 160^2 town (35,840 voxels) 0.86 -> 0.28 ms, 512^2 city 9.2 -> 3.0.
 #include "sgb_internal.cuh"
 
 namespace sgb {
 namespace {
 
-constexpr int kEncWarps = 4;        // large instance
+constexpr int kEncWarps = 4;        // the two passes for long lists
 constexpr int kIdsCap = 4096;
 constexpr int kRunsCap = 2624;
-constexpr int kSmallWarps = 8;      // small instance
-constexpr int kSmallIds = 1024;
+constexpr int kSmallIds = 1024;     // lists encoded in registers
+constexpr int kCopyWarps = 8;
 constexpr int kW4 = 0, kEnd = 7;
 
 __device__ __forceinline__ int width_class(uint32_t x)
@@ -142,25 +158,268 @@ __device__ int load_sorted(const int* row, int k, uint32_t* ids, int lane, bool 
     return n2;
 }
 
-// Two instances per pass: the small one (lists <= kSmallIds ids, 8 KB of
-// shared memory per warp, 8 warps per block) takes almost every voxel; the
-// large one takes only the longer lists (up to one id per direction).
-template <int IDS, int RUNS, int WARPS, bool LARGE>
+// ---- lists of up to kSmallIds ids -------------------------------------------------
+
+constexpr unsigned kAll = 0xFFFFFFFFu;
+
+// Bytes of the longest stream of k ids, and its room (whole 16-byte pieces).
+__host__ __device__ constexpr int stream_bytes(int k) { return 4 * k + k + 3 * ((k + 7) / 8); }
+__host__ __device__ constexpr int stream_room(int k) { return (stream_bytes(k) + 15) / 16 * 16; }
+// Where the stream of a list of k ids starts in its row (in ints).
+__device__ __forceinline__ int stream_at(int k) { return (k + 3) & ~3; }
+
+__device__ __forceinline__ void swap_desc(uint32_t& a, uint32_t& b)
+{
+    const uint32_t hi = max(a, b), lo = min(a, b);
+    a = hi;
+    b = lo;
+}
+
+// Sorts 32 E ids descending, lane l holding the places [l E, (l + 1) E).  Every
+// merge starts with a mirrored step, so all comparisons point the same way.
+template <int E>
+__device__ __forceinline__ void sort_desc(uint32_t (&x)[E], int lane)
+{
+#pragma unroll
+    for (int size = 2; size <= 32 * E; size <<= 1) {
+        if (size <= E) {
+#pragma unroll
+            for (int j = 0; j < E; ++j) {
+                const int m = (j & ~(size - 1)) + size - 1 - (j & (size - 1));
+                if (j < m) swap_desc(x[j], x[m]);
+            }
+        } else {
+            const int lanes = size / E;
+            const bool upper = (lane & (lanes >> 1)) != 0;
+#pragma unroll
+            for (int j = 0; j < E / 2; ++j) {
+                const uint32_t a = __shfl_xor_sync(kAll, x[E - 1 - j], lanes - 1);
+                const uint32_t b = __shfl_xor_sync(kAll, x[j], lanes - 1);
+                x[j] = upper ? min(x[j], a) : max(x[j], a);
+                x[E - 1 - j] = upper ? min(x[E - 1 - j], b) : max(x[E - 1 - j], b);
+            }
+        }
+#pragma unroll
+        for (int stride = size >> 2; stride > 0; stride >>= 1) {
+            if (stride >= E) {
+                const bool upper = (lane & (stride / E)) != 0;
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                    const uint32_t a = __shfl_xor_sync(kAll, x[j], stride / E);
+                    x[j] = upper ? min(x[j], a) : max(x[j], a);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < E; ++j)
+                    if ((j & stride) == 0) swap_desc(x[j], x[j + stride]);
+            }
+        }
+    }
+}
+
+// Encodes k ids (sorted, as sort_desc leaves them) into st; pieces: k words.
+// Returns the stream's bytes.
+template <int E>
+__device__ __forceinline__ int encode_sorted(uint32_t (&x)[E], int k, unsigned char* st, uint32_t* pieces, int lane)
+{
+    constexpr int kNone = 15;   // class past the list's end
+    const int base = lane * E, n = min(max(k - base, 0), E);   // this lane's ids
+    const uint32_t before = __shfl_up_sync(kAll, x[E - 1], 1);
+#pragma unroll
+    for (int j = E - 1; j > 0; --j) x[j] = x[j - 1] - x[j];
+    if (lane > 0) x[0] = before - x[0];   // x: deltas from here on
+    int w[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) w[j] = j < n ? width_class(x[j]) : kNone;
+    // ids that join the wider run before them
+    int wl = __shfl_up_sync(kAll, w[E - 1], 1), wr = __shfl_down_sync(kAll, w[0], 1);
+    if (lane == 0) wl = kNone;
+    if (lane == 31) wr = kNone;
+    unsigned c = 0;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        const int l = j ? w[j - 1] : wl, r = j + 1 < E ? w[j + 1] : wr;
+        if (l == w[j] + 1 && r != w[j] && l < kNone) c |= 1u << j;
+    }
+    const unsigned cl = __shfl_up_sync(kAll, c, 1);
+    const auto at = [&](int j) { return ((cl >> j) & 1u) != 0; };
+    bool joined = lane > 0 && at(E - 1) && !(at(E - 2) && !(at(E - 3) && !at(E - 4)));
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        joined = ((c >> j) & 1u) != 0 && !joined;
+        if (joined) ++w[j];
+    }
+    // starts of runs
+    wl = __shfl_up_sync(kAll, w[E - 1], 1);
+    if (lane == 0) wl = kNone;
+    int start = -1;
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+        if (w[j] != (j ? w[j - 1] : wl)) start = base + j;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, start, o);
+        if (lane >= o) start = max(start, y);
+    }
+    start = __shfl_up_sync(kAll, start, 1);   // the last start before this lane (lane 0 has one of its own)
+    // pieces: runs split every 255 ids; two 4-bit deltas share a byte
+    unsigned first = 0, odd = 0;
+    int bytes = 0;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        if (w[j] != (j ? w[j - 1] : wl)) start = base + j;
+        int rel = base + j - start;
+        while (rel >= 255) rel -= 255;
+        if (j < n) {
+            if (rel == 0) first |= 1u << j;
+            if (rel & 1) odd |= 1u << j;
+            bytes += w[j] ? w[j] : 1 - (rel & 1);
+        }
+    }
+    int sum = bytes | (__popc(first) << 16);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, sum, o);
+        if (lane >= o) sum += y;
+    }
+    const int total = __shfl_sync(kAll, sum, 31), np = total >> 16, payload = total & 0xFFFF;
+    sum -= bytes | (__popc(first) << 16);
+    int b = sum & 0xFFFF, p = (sum >> 16) - 1;   // bytes before this id, its piece
+    const uint32_t xr = __shfl_down_sync(kAll, x[0], 1);
+    const int apart = __shfl_down_sync(kAll, (n == 0 || (first & 1u)) ? 1 : 0, 1);
+    const bool ends = lane == 31 || apart != 0;   // the next lane's first id is in another piece, or past the end
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+        if (j >= n) break;
+        if ((first >> j) & 1u) {
+            ++p;
+            pieces[p] = ((uint32_t)b << 14) | (uint32_t)((base + j) << 3) | (uint32_t)w[j];
+        }
+        // blocks of 8 pieces: 3 bytes of codes and the lengths come before a piece's payload
+        const int q = (p >> 3) + 1;
+        unsigned char* d = st + b + 3 * q + min(np, 8 * q);
+        if (w[j] == kW4) {
+            if (((odd >> j) & 1u) == 0) {
+                const bool alone = j + 1 < E ? (j + 1 >= n || ((first >> (j + 1)) & 1u)) : ends;
+                const uint32_t y = j + 1 < E ? x[j + 1] : xr;
+                *d = (unsigned char)((x[j] << 4) | (alone ? 0u : y & 0x0Fu));
+                ++b;
+            }
+        } else {
+            for (int i = 0; i < w[j]; ++i) d[i] = (unsigned char)(x[j] >> (8 * (w[j] - 1 - i)));
+            b += w[j];
+        }
+    }
+    __syncwarp();
+    for (int p0 = 0; p0 < np; p0 += 32) {
+        const int i = p0 + lane;
+        const uint32_t pc = i < np ? pieces[i] : 0u;
+        const int next = i + 1 < np ? (int)((pieces[i + 1] >> 3) & 0x7FFu) : k;
+        const int q = i >> 3, j = i & 7;
+        unsigned char* blk = st + (__shfl_sync(kAll, pc, lane & ~7) >> 14) + 11 * q;
+        uint32_t bits = (i < np ? pc & 7u : (uint32_t)kEnd) << ((7 - j) * 3);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) bits |= __shfl_xor_sync(kAll, bits, o);
+        if (i < np) blk[3 + j] = (unsigned char)(next - (int)((pc >> 3) & 0x7FFu));
+        if (j < 3 && 8 * q < np) blk[j] = (unsigned char)(bits >> (16 - 8 * j));
+    }
+    __syncwarp();
+    return payload + np + 3 * ((np + 7) / 8);
+}
+
+// The list of a row, a lane's ids side by side: sorted, written back, encoded.
+template <int E>
+__device__ __forceinline__ int encode_row(int* row, int k, unsigned char* st, uint32_t* pieces, int lane)
+{
+    uint32_t x[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) x[j] = 32 * j + lane < k ? (uint32_t)row[32 * j + lane] : 0u;
+    sort_desc<E>(x, lane);
+#pragma unroll
+    for (int j = 0; j < E / 4; ++j) {   // whole pieces: the stream starts on the next one
+        const int i = lane * E + 4 * j;
+        if (i < k) *reinterpret_cast<uint4*>(row + i) = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+    }
+    return encode_sorted<E>(x, k, st, pieces, lane);
+}
+
+// Lists of (E == 16) up to 512, (E == 32) 513 to 1024 ids: size of the stream,
+// which is left in the row after the sorted list.
+template <int E, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
+k_barle_encode(int chunk_count, int D, int* __restrict__ raw, const int* __restrict__ counts, int* __restrict__ sizes,
+               int* __restrict__ err, const int* __restrict__ perm)
+{
+    __shared__ __align__(16) unsigned char s_stream[WARPS][stream_room(32 * E)];
+    __shared__ uint32_t s_pieces[WARPS][32 * E];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int lv = blockIdx.x * WARPS + warp;   // row
+    if (lv >= chunk_count) return;
+    const int u = perm ? perm[lv] : lv;         // voxel of the row
+    const int k = counts[u];
+    if (E == 32 ? k <= 512 || k > 1024 : k > 512) return;
+    if (E == 16 && k <= 0) {
+        if (lane == 0) sizes[u] = 0;
+        return;
+    }
+    if (k > D) {
+        if (lane == 0) {
+            sizes[u] = 0;
+            atomicOr(err, kErrListCapacity);
+        }
+        return;
+    }
+    int* row = raw + (size_t)lv * D;
+    unsigned char* st = s_stream[warp];
+    const int size = E == 16 && k <= 256 ? encode_row<8>(row, k, st, s_pieces[warp], lane)
+                                         : encode_row<E>(row, k, st, s_pieces[warp], lane);
+    if (lane == 0) sizes[u] = size;
+    uint4* dst = reinterpret_cast<uint4*>(row + stream_at(k));
+    for (int i = lane; i < (size + 15) / 16; i += 32) dst[i] = reinterpret_cast<const uint4*>(st)[i];
+}
+
+// The streams of k_barle_encode to their places: whole words there, from pairs
+// of words here.
+__global__ void __launch_bounds__(kCopyWarps * 32)
+k_barle_copy(int chunk_count, int D, const int* __restrict__ raw, const int* __restrict__ counts,
+             const long long* __restrict__ offsets, unsigned char* __restrict__ out, const int* __restrict__ inv)
+{
+    const int lane = threadIdx.x & 31;
+    const int lv = blockIdx.x * kCopyWarps + (threadIdx.x >> 5);
+    if (lv >= chunk_count) return;
+    const int k = counts[lv];
+    if (k <= 0 || k > kSmallIds) return;
+    const long long o = offsets[lv];
+    const int size = (int)(offsets[lv + 1] - o);
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(raw + (size_t)(inv ? inv[lv] : lv) * D + stream_at(k));
+    unsigned char* dst = out + o;
+    const int head = min(size, (int)((0u - (unsigned)reinterpret_cast<uintptr_t>(dst)) & 3u));
+    const int words = (size - head) >> 2, tail = size - head - 4 * words;
+    if (lane < head) dst[lane] = (unsigned char)(src[0] >> (8 * lane));
+    uint32_t* dw = reinterpret_cast<uint32_t*>(dst + head);
+    for (int i = lane; i < words; i += 32) dw[i] = __funnelshift_r(src[i], src[i + 1], 8 * head);   // head = 0: src[i]
+    if (lane < tail) {
+        const int at = size - tail + lane;
+        dst[at] = (unsigned char)(src[at >> 2] >> (8 * (at & 3)));
+    }
+}
+
+// ---- longer lists -----------------------------------------------------------------
+
+__global__ void __launch_bounds__(kEncWarps * 32)
 k_barle_size(int chunk_count, int D, int* __restrict__ raw, const int* __restrict__ counts,
              int* __restrict__ sizes, int* __restrict__ err, const int* __restrict__ perm)
 {
     extern __shared__ uint32_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t* ids = smem + warp * (IDS + RUNS);
-    uint32_t* runs = ids + IDS;
-    const int lv = blockIdx.x * WARPS + warp;   // row
+    uint32_t* ids = smem + warp * (kIdsCap + kRunsCap);
+    uint32_t* runs = ids + kIdsCap;
+    const int lv = blockIdx.x * kEncWarps + warp;   // row
     if (lv >= chunk_count) return;
     const int u = perm ? perm[lv] : lv;          // voxel of the row
     const int k = counts[u];
-    if (LARGE != (k > kSmallIds)) return;
-    if (k <= 0) { if (lane == 0) sizes[u] = 0; return; }
-    if (k > D || k > RUNS) { if (lane == 0) { sizes[u] = 0; atomicOr(err, kErrListCapacity); } return; }
+    if (k <= kSmallIds) return;
+    if (k > D || k > kRunsCap) { if (lane == 0) { sizes[u] = 0; atomicOr(err, kErrListCapacity); } return; }
     int* row = raw + (size_t)lv * D;
     load_sorted(row, k, ids, lane, true);
     for (int i = lane; i < k; i += 32) row[i] = (int)ids[i];   // keep the sorted list for the write pass
@@ -188,21 +447,20 @@ k_barle_size(int chunk_count, int D, int* __restrict__ raw, const int* __restric
     if (lane == 0) sizes[u] = 3 * ((pieces + 7) / 8) + pieces + payload;
 }
 
-template <int IDS, int RUNS, int WARPS, bool LARGE>
-__global__ void __launch_bounds__(WARPS * 32)
+__global__ void __launch_bounds__(kEncWarps * 32)
 k_barle_write(int chunk_count, int D, const int* __restrict__ raw, const int* __restrict__ counts,
               const long long* __restrict__ offsets, unsigned char* __restrict__ out,
               int* __restrict__ err, const int* __restrict__ inv)
 {
     extern __shared__ uint32_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t* ids = smem + warp * (IDS + RUNS);
-    uint32_t* runs = ids + IDS;
-    const int lv = blockIdx.x * WARPS + warp;
+    uint32_t* ids = smem + warp * (kIdsCap + kRunsCap);
+    uint32_t* runs = ids + kIdsCap;
+    const int lv = blockIdx.x * kEncWarps + warp;
     if (lv >= chunk_count) return;
     const int k = counts[lv];
-    if (LARGE != (k > kSmallIds)) return;
-    if (k <= 0 || k > D || k > RUNS) return;
+    if (k <= kSmallIds) return;
+    if (k > D || k > kRunsCap) return;
     const int* row = raw + (size_t)(inv ? inv[lv] : lv) * D;
     load_sorted(row, k, ids, lane, false);   // already sorted by k_barle_size
     // the runs k_barle_size left after the list, else built again
@@ -277,40 +535,22 @@ k_barle_write(int chunk_count, int D, const int* __restrict__ raw, const int* __
 
 }  // namespace
 
-template <int IDS, int RUNS, int WARPS, bool LARGE>
-cudaError_t size_pass(int chunk_count, int D, int* raw, const int* counts, int* sizes, int* err, const int* perm,
-                      cudaStream_t st)
-{
-    const size_t smem = (size_t)WARPS * (IDS + RUNS) * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute(k_barle_size<IDS, RUNS, WARPS, LARGE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_barle_size<IDS, RUNS, WARPS, LARGE><<<(chunk_count + WARPS - 1) / WARPS, WARPS * 32, smem, st>>>(
-        chunk_count, D, raw, counts, sizes, err, perm);
-    return cudaGetLastError();
-}
-
-template <int IDS, int RUNS, int WARPS, bool LARGE>
-cudaError_t write_pass(int chunk_count, int D, const int* raw, const int* counts, const long long* offsets,
-                       unsigned char* out, int* err, const int* inv, cudaStream_t st)
-{
-    const size_t smem = (size_t)WARPS * (IDS + RUNS) * sizeof(uint32_t);
-    cudaError_t e = cudaFuncSetAttribute(k_barle_write<IDS, RUNS, WARPS, LARGE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_barle_write<IDS, RUNS, WARPS, LARGE><<<(chunk_count + WARPS - 1) / WARPS, WARPS * 32, smem, st>>>(
-        chunk_count, D, raw, counts, offsets, out, err, inv);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_barle_size(int chunk_count, int D, int* raw, const int* counts, int* sizes, int* err,
                               const int* perm, cudaStream_t st)
 {
     if (chunk_count <= 0) return cudaSuccess;
-    cudaError_t e = size_pass<kSmallIds, kSmallIds, kSmallWarps, false>(chunk_count, D, raw, counts, sizes, err,
-                                                                        perm, st);
+    // a row holds the list and the stream of up to kSmallIds ids, and starts on 16 bytes
+    if (D % 4 != 0 || 4 * D < 4 * kSmallIds + stream_room(kSmallIds)) return cudaErrorInvalidValue;
+    k_barle_encode<16, 8><<<(chunk_count + 7) / 8, 8 * 32, 0, st>>>(chunk_count, D, raw, counts, sizes, err, perm);
+    k_barle_encode<32, 4><<<(chunk_count + 3) / 4, 4 * 32, 0, st>>>(chunk_count, D, raw, counts, sizes, err, perm);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return size_pass<kIdsCap, kRunsCap, kEncWarps, true>(chunk_count, D, raw, counts, sizes, err, perm, st);
+    constexpr size_t smem = (size_t)kEncWarps * (kIdsCap + kRunsCap) * sizeof(uint32_t);
+    e = cudaFuncSetAttribute(k_barle_size, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_barle_size<<<(chunk_count + kEncWarps - 1) / kEncWarps, kEncWarps * 32, smem, st>>>(chunk_count, D, raw, counts,
+                                                                                         sizes, err, perm);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_barle_write(int chunk_count, int D, const int* raw, const int* counts,
@@ -318,10 +558,16 @@ cudaError_t launch_barle_write(int chunk_count, int D, const int* raw, const int
                                cudaStream_t st)
 {
     if (chunk_count <= 0) return cudaSuccess;
-    cudaError_t e = write_pass<kSmallIds, kSmallIds, kSmallWarps, false>(chunk_count, D, raw, counts, offsets,
-                                                                         out, err, inv, st);
+    k_barle_copy<<<(chunk_count + kCopyWarps - 1) / kCopyWarps, kCopyWarps * 32, 0, st>>>(chunk_count, D, raw, counts,
+                                                                                         offsets, out, inv);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return write_pass<kIdsCap, kRunsCap, kEncWarps, true>(chunk_count, D, raw, counts, offsets, out, err, inv, st);
+    constexpr size_t smem = (size_t)kEncWarps * (kIdsCap + kRunsCap) * sizeof(uint32_t);
+    e = cudaFuncSetAttribute(k_barle_write, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_barle_write<<<(chunk_count + kEncWarps - 1) / kEncWarps, kEncWarps * 32, smem, st>>>(
+        chunk_count, D, raw, counts, offsets, out, err, inv);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_barle_size(int chunk_count, int D, int* raw, const int* counts,
