@@ -6,8 +6,8 @@
 // result.  For each group of directions this file builds one table over the
 // bordered grid,
 //
-//     bound[cell] = min(maxz, max of the heights of every cell a ray of the
-//                   group can visit from `cell` on),
+//     bound[cell] = min(maxz, max of the heights of every block of 2 x 2 cells a ray
+//                   of the group can visit from a cell of `cell`'s block on),
 //
 // and the tracer ends an upward ray with no hit when its height exceeds the
 // bound of a cell it has reached (it loads the bound of the cell a group of
@@ -29,8 +29,12 @@
 // L crossings, so every visited cell lies within eps of that line at the same
 // time.  The cells from the current cell c on therefore lie in
 // c + (-1 - 2 eps, 1 + 2 eps]^2 + K, where K is any closed cone containing
-// (1/dX, 1/dY).  K is taken between two consecutive primitive vectors a, b
-// of the Farey set of order 8 (all primitive (p, q) with p, q <= 8, sorted by
+// (1/dX, 1/dY).  Divided by 2, with c at any place f in [0, 1)^2 of its block and
+// a cell anywhere in its own, the blocks from c's block B on lie in
+// B + (-1 - q, 1 + q)^2 + K, q = (1 + 2 eps) / 2: the same cone (it has no scale) and
+// a box that replaces 1 + 2 eps by 1 + q.
+//
+// K is taken between two consecutive primitive vectors a, b of the Farey set of order 4 (all primitive (p, q) with p, q <= 4, sorted by
 // angle), so det(a, b) = 1 and the lattice points of K are exactly the
 // non-negative combinations of a and b.  Then
 //   M(c)     = max(h(c), M(c + a), M(c + b))      (max over c + K)
@@ -39,12 +43,20 @@
 // lattice point e = p - frac_ab(p), frac_ab(p) in {s a + t b : s, t in [0,1)};
 // so the bound is the maximum of M over the window
 //   e_X in [-(r + a_X + b_X), r],  e_Y in [-(r + a_Y + b_Y), r],
-//   r = 1 + ceil(2 eps),
-// taken as two one-dimensional passes.  Window apexes past the grid's far
-// sides (in unsigned coordinates) reach no cell and are skipped; an apex
-// before its near sides would need M outside the grid, so the bound there is
-// +inf (the range test alone, as the reference).  Non-finite heights: NaN
-// never hits and fmaxf skips it; +inf enters the maximum as itself.
+//   r = 1 + ceil(q),
+// taken as two one-dimensional passes.  All of it runs over the blocks with a
+// margin of r + 8 on every side (heights -inf), so that every apex of a block's
+// window has its M.  A ray off the grid hits nothing more, so the bound there may
+// be anything; the tables have +inf on the border.  Non-finite heights: NaN never
+// hits and fmaxf skips it; +inf enters the maximum as itself.
+//
+// Bound: latency of the lines (a thread follows one line of blocks), launches, and
+// the bytes of the tables per cell (0.3 GB at 1024^2, which the tracer reads with the
+// index it has anyway; reading them by block cost it 4 ms there).  Built per cell,
+// with cones of order 8, they took 2.9 ms of a 1024^2 run and 64 us of a 64^2 one.
+// Trace stage then, with blocks of 4 x 4 and order 8, 4 x 4 and order 4, 2 x 2 and order 4: 1024^2
+// 44.6, 44.5, 44.2, 43.9 ms; 512^2 10.75, 10.60, 10.52, 10.44; 160^2 0.99, 0.91, 0.90, 0.90; 64^2
+// 0.248, 0.229, 0.215, 0.220.
 #include "sgb_internal.cuh"
 
 #include <climits>
@@ -53,10 +65,8 @@
 namespace sgb {
 namespace {
 
-__device__ __forceinline__ size_t pad_index(int x, int y, int W)
-{
-    return (size_t)(x + 1) + (size_t)(y + 1) * (size_t)(W + 2);
-}
+// W and H below are those of the blocks with their margins.
+__device__ __forceinline__ size_t block_index(int x, int y, int W) { return (size_t)y * W + x; }
 
 __device__ __forceinline__ void to_grid(const ConeSpec& c, int X, int Y, int W, int H, int& x, int& y)
 {
@@ -64,10 +74,24 @@ __device__ __forceinline__ void to_grid(const ConeSpec& c, int X, int Y, int W, 
     y = c.sy > 0 ? Y : H - 1 - Y;
 }
 
+// Heights of the blocks, -inf in the margins.
+__global__ void k_cone_blocks(const float* __restrict__ grid, int gw, int gh, int margin, int W, int H,
+                              float* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= W * H) return;
+    const int y = i / W, x = i - y * W;
+    const int cx = (x - margin) << kConeShift, cy = (y - margin) << kConeShift;
+    float m = -__int_as_float(0x7f800000);
+    for (int v = max(cy, 0); v < min(cy + (1 << kConeShift), gh); ++v)
+        for (int u = max(cx, 0); u < min(cx + (1 << kConeShift), gw); ++u) m = fmaxf(m, __ldg(grid + (size_t)v * gw + u));
+    out[i] = m;
+}
+
 // Suffix maxima along the lattice lines of one cone vector (u, v) (unsigned
 // coordinates): dst(c) = max(src(c), dst(c + (u, v))).  One thread a line,
 // started at the line's last cell inside the grid (c + (u, v) outside).
-// PASS 0: src = the grid's heights ([H][W]);  PASS 1: src = a bordered table.
+// PASS 0: src = the blocks' heights;  PASS 1: src = a table.
 template <int PASS>
 __global__ void k_cone_lines(const float* __restrict__ src, int W, int H, const ConeSpec* __restrict__ specs,
                              float* __restrict__ dst, size_t stride)
@@ -86,18 +110,18 @@ __global__ void k_cone_lines(const float* __restrict__ src, int W, int H, const 
     // a known trip count lets the loads of an unrolled stretch issue together
     const int n = min(u > 0 ? X / u : INT_MAX, v > 0 ? Y / v : INT_MAX) + 1;
     float m = -__int_as_float(0x7f800000);
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 0; i < n; ++i, X -= u, Y -= v) {
         int x, y;
         to_grid(c, X, Y, W, H, x, y);
-        const size_t p = pad_index(x, y, W);
-        m = fmaxf(m, in[PASS == 0 ? (size_t)y * W + x : p]);
+        const size_t p = block_index(x, y, W);
+        m = fmaxf(m, in[p]);
         out[p] = m;
     }
 }
 
 // Window maxima of M: PASS 0 over X offsets, PASS 1 over Y offsets (then
-// min with maxz); both read src and write dst (bordered tables).  A block
+// min with maxz); both read src and write dst (tables).  A block
 // stages the stretch of its rows (PASS 0: 256 cells of one row; PASS 1: 64
 // rows of 32 columns) plus the window's reach in shared memory, cells past
 // the grid as -inf (a window clipped at the grid's edge), and each cell
@@ -119,24 +143,21 @@ k_cone_window(int W, int H, float maxz, int r, const ConeSpec* __restrict__ spec
     const int s = PASS == 0 ? c.sx : c.sy;
     const int lo = s > 0 ? -back : -r, hi = s > 0 ? r : back;
     const int width = hi - lo + 1;
-    const float ninf = -__int_as_float(0x7f800000), pinf = __int_as_float(0x7f800000);
+    const float ninf = -__int_as_float(0x7f800000);
     if (PASS == 0) {
         const int segs = (W + kWinRow - 1) / kWinRow;
         const int y = (int)(blockIdx.x / segs), x0 = (int)(blockIdx.x % segs) * kWinRow;
         const int n = kWinRow + width - 1;
         for (int j = threadIdx.x; j < n; j += blockDim.x) {
             const int q = x0 + lo + j;
-            span[j] = (q >= 0 && q < W) ? in[pad_index(q, y, W)] : ninf;
+            span[j] = (q >= 0 && q < W) ? in[block_index(q, y, W)] : ninf;
         }
         __syncthreads();
         const int x = x0 + (int)threadIdx.x;
         if (x >= W) return;
-        // the window's near end (unsigned offset -(r + a + b)) must lie inside
-        const bool open = s > 0 ? x + lo < 0 : x + hi > W - 1;
-        float m = open ? pinf : ninf;
-        if (!open)
-            for (int j = 0; j < width; ++j) m = fmaxf(m, span[threadIdx.x + j]);
-        out[pad_index(x, y, W)] = m;
+        float m = ninf;
+        for (int j = 0; j < width; ++j) m = fmaxf(m, span[threadIdx.x + j]);
+        out[block_index(x, y, W)] = m;
     } else {
         const int cols = (W + kWinCols - 1) / kWinCols;
         const int x0 = (int)(blockIdx.x % cols) * kWinCols, y0 = (int)(blockIdx.x / cols) * kWinRows;
@@ -145,65 +166,85 @@ k_cone_window(int W, int H, float maxz, int r, const ConeSpec* __restrict__ spec
         const int rows = kWinRows + width - 1;
         for (int j = ty; j < rows; j += blockDim.x / kWinCols) {
             const int q = y0 + lo + j;
-            span[j * kWinCols + tx] = (x < W && q >= 0 && q < H) ? in[pad_index(x, q, W)] : ninf;
+            span[j * kWinCols + tx] = (x < W && q >= 0 && q < H) ? in[block_index(x, q, W)] : ninf;
         }
         __syncthreads();
         if (x >= W) return;
         for (int k = 0; k < kWinRowsPerThread; ++k) {
             const int yl = ty * kWinRowsPerThread + k, y = y0 + yl;
             if (y >= H) break;
-            const bool open = s > 0 ? y + lo < 0 : y + hi > H - 1;
-            float m = open ? pinf : ninf;
-            if (!open)
-                for (int j = 0; j < width; ++j) m = fmaxf(m, span[(yl + j) * kWinCols + tx]);
-            out[pad_index(x, y, W)] = fminf(maxz, m);
+            float m = ninf;
+            for (int j = 0; j < width; ++j) m = fmaxf(m, span[(yl + j) * kWinCols + tx]);
+            out[block_index(x, y, W)] = fminf(maxz, m);
         }
     }
 }
 
-// The border cells of every table: +inf (a ray there stops on the height
-// test of the bordered heightmap, never on its bound).
-__global__ void k_cone_border(int W, int H, float* __restrict__ tabs, size_t stride)
+// The blocks' bounds to the cells of the bordered tables, kExpand tables a block.
+constexpr int kExpand = 8;
+
+__global__ void __launch_bounds__(256)
+k_cone_cells(const float* __restrict__ src, size_t blocks, int W, int margin, int gw, int gh, int n_specs,
+             float* __restrict__ tabs, size_t stride)
 {
-    const int Wp = W + 2;
+    const int Wp = gw + 2;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2LL * (Wp + H)) return;
-    size_t p;
-    if (i < Wp)                p = (size_t)i;                                     // top row
-    else if (i < 2 * Wp)       p = (size_t)(i - Wp) + (size_t)(H + 1) * Wp;       // bottom row
-    else if (i < 2 * Wp + H)   p = (size_t)(i - 2 * Wp + 1) * Wp;                 // left column
-    else                       p = (size_t)(i - 2 * Wp - H + 1) * Wp + (Wp - 1);  // right column
-    tabs[stride * blockIdx.y + p] = __int_as_float(0x7f800000);
+    if (i >= (long long)Wp * (gh + 2)) return;
+    const int y = (int)(i / Wp), x = (int)(i - (long long)y * Wp);
+    const bool in = x > 0 && x <= gw && y > 0 && y <= gh;
+    // a border cell's block may be the margin's first one
+    const size_t from = block_index(((x - 1) >> kConeShift) + margin, ((y - 1) >> kConeShift) + margin, W);
+    const int t0 = blockIdx.y * kExpand, n = min(kExpand, n_specs - t0);
+    float v[kExpand];
+#pragma unroll
+    for (int t = 0; t < kExpand; ++t) v[t] = t < n ? __ldg(src + blocks * (t0 + t) + from) : 0.0f;
+#pragma unroll
+    for (int t = 0; t < kExpand; ++t)
+        if (t < n) tabs[stride * (t0 + t) + i] = in ? v[t] : __int_as_float(0x7f800000);
 }
 
 }  // namespace
 
-int cone_window_radius(int W, int H)
+static int cone_window_radius(int W, int H)
 {
     const double L = (double)(W > H ? W : H) + 4.0;
     const double eps2 = 2.0 * L * (L + 1.0) / 16777216.0;
-    return 1 + (int)std::ceil(eps2);
+    return 1 + (int)std::ceil((1.0 + eps2) / (1 << kConeShift));
 }
 
-cudaError_t launch_cone_tables(const float* grid, int W, int H, float maxz, const ConeSpec* specs, int n_specs,
+static int cone_margin(int W, int H) { return cone_window_radius(W, H) + 2 * kConeOrder; }
+static int cone_blocks(int cells, int margin) { return ((cells + (1 << kConeShift) - 1) >> kConeShift) + 2 * margin; }
+
+size_t cone_scratch(int W, int H, int n_specs)
+{
+    const int margin = cone_margin(W, H);
+    return (size_t)cone_blocks(W, margin) * cone_blocks(H, margin) * (2 * (size_t)n_specs + 1);
+}
+
+cudaError_t launch_cone_tables(const float* grid, int gw, int gh, float maxz, const ConeSpec* specs, int n_specs,
                                float* tabs, float* tmp, size_t stride, cudaStream_t st)
 {
-    if (W <= 0 || H <= 0 || n_specs <= 0) return cudaSuccess;
-    const unsigned border = (unsigned)((2LL * (W + 2 + H) + 255) / 256);
-    // start cells of a line family: at most kConeOrder (W + H)
+    if (gw <= 0 || gh <= 0 || n_specs <= 0) return cudaSuccess;
+    const int r = cone_window_radius(gw, gh), margin = cone_margin(gw, gh);
+    const int W = cone_blocks(gw, margin), H = cone_blocks(gh, margin);
+    const size_t blocks = (size_t)W * H;
+    float *base = tmp, *a = base + blocks, *b = a + blocks * n_specs;
+    // start blocks of a line family: at most kConeOrder (W + H)
     const unsigned lines = (unsigned)(((long long)kConeOrder * (W + H) + 255) / 256);
-    const int r = cone_window_radius(W, H);
-    k_cone_lines<0><<<dim3(lines, n_specs), 256, 0, st>>>(grid, W, H, specs, tmp, stride);
-    k_cone_lines<1><<<dim3(lines, n_specs), 256, 0, st>>>(tmp, W, H, specs, tabs, stride);
+    k_cone_blocks<<<(unsigned)((blocks + 255) / 256), 256, 0, st>>>(grid, gw, gh, margin, W, H, base);
+    k_cone_lines<0><<<dim3(lines, n_specs), 256, 0, st>>>(base, W, H, specs, a, blocks);
+    k_cone_lines<1><<<dim3(lines, n_specs), 256, 0, st>>>(a, W, H, specs, b, blocks);
     // the widest window: r on one side, r + a + b (components <= kConeOrder each) on the other
     const int wmax = 2 * r + 2 * kConeOrder + 1;
     const unsigned win0 = (unsigned)(((long long)W + kWinRow - 1) / kWinRow * H);
     const unsigned win1 = (unsigned)(((long long)W + kWinCols - 1) / kWinCols * ((H + kWinRows - 1) / kWinRows));
-    k_cone_window<0><<<dim3(win0, n_specs), 256, sizeof(float) * (kWinRow + wmax), st>>>(W, H, maxz, r, specs,
-                                                                                       tabs, tmp, stride);
-    k_cone_window<1><<<dim3(win1, n_specs), 256, sizeof(float) * kWinCols * (kWinRows + wmax), st>>>(
-        W, H, maxz, r, specs, tmp, tabs, stride);
-    k_cone_border<<<dim3(border, n_specs), 256, 0, st>>>(W, H, tabs, stride);
+    k_cone_window<0><<<dim3(win0, n_specs), 256, sizeof(float) * (kWinRow + wmax), st>>>(W, H, maxz, r, specs, b, a,
+                                                                                       blocks);
+    k_cone_window<1><<<dim3(win1, n_specs), 256, sizeof(float) * kWinCols * (kWinRows + wmax), st>>>(W, H, maxz, r,
+                                                                                                 specs, a, b, blocks);
+    const size_t cells = (size_t)(gw + 2) * (gh + 2);
+    k_cone_cells<<<dim3((unsigned)((cells + 255) / 256), (n_specs + kExpand - 1) / kExpand), 256, 0, st>>>(
+        b, blocks, W, margin, gw, gh, n_specs, tabs, stride);
     return cudaGetLastError();
 }
 

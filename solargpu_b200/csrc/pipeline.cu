@@ -417,10 +417,11 @@ int padded_grid(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables&
         if (std::atoi(env) == 0) nt = 0;
     DevBuf& tabs = c->cone_shared ? *c->cone_shared : c->cone;
     const size_t bytes = sizeof(float) * cells * (size_t)nt;
-    const bool scratch_in_raw = c->raw.cap >= bytes;
+    const size_t scratch = sizeof(float) * cone_scratch(W, H, nt);
+    const bool scratch_in_raw = c->raw.cap >= scratch;
     // device memory these tables would add to what the context holds
     const size_t grow = (bytes > tabs.cap ? bytes - tabs.cap : 0) +
-                        (!scratch_in_raw && bytes > c->cone_tmp.cap ? bytes - c->cone_tmp.cap : 0);
+                        (!scratch_in_raw && scratch > c->cone_tmp.cap ? scratch - c->cone_tmp.cap : 0);
     if (nt > 0 && grow > 0) {
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
@@ -437,7 +438,7 @@ int padded_grid(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables&
     c->launches += 1;
     if (nt == 0) return SOLAR_GPU_OK;
     if (ensure(c, tabs, bytes) != SOLAR_GPU_OK ||
-        (!scratch_in_raw && ensure(c, c->cone_tmp, bytes) != SOLAR_GPU_OK)) {
+        (!scratch_in_raw && ensure(c, c->cone_tmp, scratch) != SOLAR_GPU_OK)) {
         (void)cudaGetLastError();   // no room after all: the tracer runs without the tables
         return SOLAR_GPU_OK;
     }
@@ -445,7 +446,7 @@ int padded_grid(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables&
     CK(cudaMemcpyAsync(c->cone_specs.p, sky.cones.data(), sizeof(ConeSpec) * nt, cudaMemcpyHostToDevice, st));
     CK(launch_cone_tables(s->grid, W, H, s->max_height, as<ConeSpec>(c->cone_specs), nt, as<float>(tabs),
                           scratch_in_raw ? as<float>(c->raw) : as<float>(c->cone_tmp), cells, st));
-    c->launches += 5;
+    c->launches += 6;
     ds.cone = as<float>(tabs);
     ds.cone_stride = cells;
     return SOLAR_GPU_OK;

@@ -40,7 +40,8 @@ struct ConeSpec {
     int sx, sy;
     int ax, ay, bx, by;
 };
-constexpr int kConeOrder = 8;        // cone vectors have components <= 8
+constexpr int kConeOrder = 4;        // cone vectors have components <= 4
+constexpr int kConeShift = 1;        // the tables are built on blocks of 2 x 2 cells
 constexpr int kMaxConeTables = 1024; // 10 bits of DirEntry::meta
 
 // Per daylight hour, FP32 values of the FP64-evaluated solar geometry.
@@ -90,10 +91,10 @@ void set_last_error(const char* msg);
 // gpad [(H + 2) * (W + 2)] = grid inside a one-cell border of +inf.
 cudaError_t launch_pad_grid(const float* grid, int W, int H, float* gpad, cudaStream_t st);
 // Early-exit tables (cone.cu): n_specs bordered tables of `stride` floats in
-// tabs; tmp holds as many (scratch).
+// tabs; tmp is scratch of cone_scratch floats.
 cudaError_t launch_cone_tables(const float* grid, int W, int H, float maxz, const ConeSpec* specs, int n_specs,
                                float* tabs, float* tmp, size_t stride, cudaStream_t st);
-int cone_window_radius(int W, int H);
+size_t cone_scratch(int W, int H, int n_specs);
 // s.gpad must be set (launch_pad_grid); s.cone may be nullptr.
 cudaError_t launch_trace(const DevScene& s, const DirEntry* dirs, int D, int words32,
                          int voxel_offset, int chunk_count, int* raw, uint32_t* shadow,
