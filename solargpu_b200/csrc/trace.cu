@@ -33,7 +33,7 @@ constexpr int kTraceBlock = 128;
 constexpr int kDirParts = 32;      // blocks per voxel block, each 1/32 of the directions (16: +0.6% at 1024^2)
 constexpr int kDedupeWarps = 4;
 constexpr int kHashSlots = 4096;   // > 2592 possible distinct hits per voxel
-constexpr int kDedupeBatch = 9;    // 2592 = 9 batches of 9 rounds of 32 directions
+constexpr int kDedupeBatch = 3;    // 2592 directions: 7 batches of 3 rounds of 128
 
 // 16 blocks of 128 threads per SM: at most 32 registers a thread, so the SM
 // holds 64 warps of rays (measured 116.4 -> 109.7 ms at 1024^2 against 38
@@ -125,14 +125,23 @@ __device__ __forceinline__ uint32_t hash_slot(uint32_t x, int bits)
 // One warp per voxel: keeps the first occurrence of each hit id in direction
 // order and compacts the row in place; counts[perm[lv]] = list length.
 //
+// Directions without a hit and hits equal to the previous direction's leave
+// first, 128 directions a round; what is left queues up in shared memory in
+// direction order and meets the hash set 32 ids at a time.
+//
 // SLOTS is the warp's shared-memory hash set.  The first pass uses a small
 // set (4 KB a warp, so many warps fit an SM) and gives up on a voxel whose
-// insert needs more than kProbes probes: it then writes nothing of the round
-// it is in and records the row in `ovf`.  Rounds before it were compacted in
-// place and the ones after it are untouched, so every entry between the
-// compacted prefix and the current round repeats an id of the prefix: the
-// second pass (4096 slots, more than the 2592 possible distinct ids) run over
-// the whole row gives the same first-occurrence list.
+// insert needs more than kProbes probes: it then writes nothing of the 32 ids
+// it is at and records the row in `ovf`.  The ids before them were compacted in
+// place; these and the later ones stand behind the compacted prefix, untouched,
+// since at least as many directions come before an id as ids.  So every other
+// entry behind the prefix repeats an id of it, and the second pass (4096
+// slots, more than the 2592 possible distinct ids) run over the whole row gives
+// the same first-occurrence list.
+//
+// Bound: instructions.  With every direction going through the set 82% of the issue
+// slots were used and the rows' bytes took a quarter of the time: 1024^2 8.82 -> 4.93
+// ms, 512^2 2.24 -> 1.25, 160^2 0.28 -> 0.17, 64^2 0.056 -> 0.037.
 constexpr int kSmallSlots = 1024;
 constexpr int kProbes = 32;   // default probe bound of the first pass (SGB_DEDUPE_PROBES overrides it)
 
@@ -147,6 +156,9 @@ k_dedupe(int chunk_count, int D, int* __restrict__ raw, int* __restrict__ counts
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     uint32_t* tab = tab_all + warp * SLOTS;
+    __shared__ int s_queue[kDedupeWarps][128 + 32];
+    int* queue = s_queue[warp];
+    const unsigned lt = (1u << lane) - 1u;
     // FIRST: row lv; else rows listed in ovf[1..ovf[0]], grid-strided
     const int w0 = blockIdx.x * kDedupeWarps + warp;
     const int nrows = FIRST ? chunk_count : ovf[0];
@@ -156,51 +168,75 @@ k_dedupe(int chunk_count, int D, int* __restrict__ raw, int* __restrict__ counts
         for (int i = lane; i < SLOTS / 4; i += 32) t4[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
         int* row = raw + (size_t)lv * D;
-        int n = 0;
-        bool gave_up = false;
-        // Rounds of 32 directions, kDedupeBatch rounds loaded ahead (they are
-        // all read before any in-place write can reach their slots).
-        for (int base = 0; base < D && !gave_up; base += 32 * kDedupeBatch) {
-            int hv[kDedupeBatch];
+        int n = 0, queued = 0, last = 0;
+        // 32 ids (0: none) against the set; the new ones are written in order.  False: it gave up.
+        const auto insert = [&](int h) {
+            const unsigned same = __match_any_sync(0xFFFFFFFFu, h);
+            const bool leader = (__ffs(same) - 1) == lane;
+            bool fresh = false, full = false;
+            if (h != 0 && leader) {
+                uint32_t slot = hash_slot((uint32_t)h, kBits);
+                const int bound = FIRST ? probes : SLOTS;
+                int probe = 0;
+                for (; probe < bound; ++probe) {
+                    const uint32_t old = atomicCAS(&tab[slot], 0u, (uint32_t)h);
+                    if (old == 0u) { fresh = true; break; }
+                    if (old == (uint32_t)h) break;
+                    slot = (slot + 1) & (SLOTS - 1);
+                }
+                full = probe == bound;
+            }
+            if (__any_sync(0xFFFFFFFFu, full)) {
+                if (lane == 0) {
+                    if (FIRST) ovf[1 + atomicAdd(ovf, 1)] = lv;
+                    else atomicOr(err, kErrHashFull);
+                }
+                return false;
+            }
+            const unsigned bal = __ballot_sync(0xFFFFFFFFu, fresh);
+            // below the directions read so far: no more ids than directions
+            if (fresh) row[n + __popc(bal & lt)] = h;
+            n += __popc(bal);
+            return true;
+        };
+        bool ok = true;
+        for (int base = 0; base < D / 4 && ok; base += 32 * kDedupeBatch) {
+            int4 hv[kDedupeBatch];
 #pragma unroll
             for (int u = 0; u < kDedupeBatch; ++u) {
                 const int d = base + 32 * u + lane;
-                hv[u] = (d < D) ? row[d] : 0;
+                hv[u] = d < D / 4 ? reinterpret_cast<const int4*>(row)[d] : make_int4(0, 0, 0, 0);
             }
 #pragma unroll
-            for (int u = 0; u < kDedupeBatch; ++u) {
-                const int h = hv[u];
-                const unsigned same = __match_any_sync(0xFFFFFFFFu, h);
-                const bool leader = (__ffs(same) - 1) == lane;
-                bool fresh = false, full = false;
-                if (h != 0 && leader) {
-                    uint32_t slot = hash_slot((uint32_t)h, kBits);
-                    const int bound = FIRST ? probes : SLOTS;
-                    int probe = 0;
-                    for (; probe < bound; ++probe) {
-                        const uint32_t old = atomicCAS(&tab[slot], 0u, (uint32_t)h);
-                        if (old == 0u) { fresh = true; break; }
-                        if (old == (uint32_t)h) break;
-                        slot = (slot + 1) & (SLOTS - 1);
-                    }
-                    full = probe == bound;
-                }
-                if (__any_sync(0xFFFFFFFFu, full)) {
-                    if (FIRST) {
-                        if (lane == 0) ovf[1 + atomicAdd(ovf, 1)] = lv;
-                    } else if (lane == 0) {
-                        atomicOr(err, kErrHashFull);
-                    }
-                    gave_up = true;
-                    break;
-                }
-                const unsigned bal = __ballot_sync(0xFFFFFFFFu, fresh);
-                // Writes land below base + 32 * (u + 1): every slot there was read.
-                if (fresh) row[n + __popc(bal & ((1u << lane) - 1u))] = h;
-                n += __popc(bal);
+            for (int u = 0; u < kDedupeBatch && ok; ++u) {
+                const int4 a = hv[u];
+                int before = __shfl_up_sync(0xFFFFFFFFu, a.w, 1);
+                if (lane == 0) before = last;
+                last = __shfl_sync(0xFFFFFFFFu, a.w, 31);
+                const bool c0 = a.x != 0 && a.x != before, c1 = a.y != 0 && a.y != a.x;
+                const bool c2 = a.z != 0 && a.z != a.y, c3 = a.w != 0 && a.w != a.z;
+                const unsigned m0 = __ballot_sync(0xFFFFFFFFu, c0), m1 = __ballot_sync(0xFFFFFFFFu, c1);
+                const unsigned m2 = __ballot_sync(0xFFFFFFFFu, c2), m3 = __ballot_sync(0xFFFFFFFFu, c3);
+                if ((m0 | m1 | m2 | m3) == 0u) continue;
+                int at = queued + __popc(m0 & lt) + __popc(m1 & lt) + __popc(m2 & lt) + __popc(m3 & lt);
+                if (c0) queue[at++] = a.x;
+                if (c1) queue[at++] = a.y;
+                if (c2) queue[at++] = a.z;
+                if (c3) queue[at] = a.w;
+                queued += __popc(m0) + __popc(m1) + __popc(m2) + __popc(m3);
+                __syncwarp();
+                int done = 0;
+                for (; ok && queued - done >= 32; done += 32) ok = insert(queue[done + lane]);
+                if (done == 0) continue;
+                queued -= done;
+                const int rest = lane < queued ? queue[done + lane] : 0;
+                __syncwarp();
+                if (lane < queued) queue[lane] = rest;
+                __syncwarp();
             }
         }
-        if (!gave_up && lane == 0) counts[perm ? perm[lv] : lv] = n;
+        if (ok && queued > 0) ok = insert(lane < queued ? queue[lane] : 0);
+        if (ok && lane == 0) counts[perm ? perm[lv] : lv] = n;
         __syncwarp();
         if (FIRST) break;
     }
