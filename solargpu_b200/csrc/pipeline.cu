@@ -115,7 +115,7 @@ struct solar_gpu_context {
         grp_cell, grp_w, w_cnt, w_off, w_tmp, w_cell, w_val, order_first, order_inv, tile_flag, tile_pos,
         tile_start, tile_union, tile_slot, tile_rows, tile_gcnt, tile_gnch, tile_gbase, tile_tbase, tile_table,
         tile_erow, tile_ew, chunk_perm, chunk_flag, chunk_pos, chunk_tmp, mma_union, mma_nch, mma_cbase,
-        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, mma_ucell, light_many, slab16, dd_ovf, vox_cnt, vox_off, vox_tmp, gpad, hour_sums, mma_retry, cone, cone_tmp, cone_specs,
+        mma_ccnt, mma_coff, mma_ent, mma_scale, mma_over, mma_ucell, light_many, slab16, dd_ovf, vox_off, gpad, hour_sums, mma_retry, cone, cone_tmp, cone_specs,
         sweep_blocks, sweep_line, box;
     int* h_scalars = nullptr;   // pinned host scratch for small read-backs
     long long mem_limit = 0;    // device bytes the buffers may hold (0: no limit)
@@ -151,7 +151,7 @@ struct solar_gpu_context {
     cudaStream_t kt_stream = nullptr;
 };
 
-static constexpr int kNumBufs = 89;
+static constexpr int kNumBufs = 87;
 extern "C" {
 static void all_bufs(solar_gpu_context* c, DevBuf** out);   // defined with the exports below
 }
@@ -1384,7 +1384,7 @@ static void all_bufs(solar_gpu_context* c, DevBuf** out)
                                 &c->chunk_pos, &c->chunk_tmp, &c->mma_union, &c->mma_nch, &c->mma_cbase,
                                 &c->mma_ccnt, &c->mma_coff, &c->mma_ent, &c->mma_scale, &c->mma_over, &c->slab16,
                                 &c->mma_ucell, &c->light_many,
-                                &c->dd_ovf, &c->vox_cnt, &c->vox_off, &c->vox_tmp, &c->gpad, &c->hour_sums, &c->mma_retry,
+                                &c->dd_ovf, &c->vox_off, &c->gpad, &c->hour_sums, &c->mma_retry,
                                 &c->cone, &c->cone_tmp, &c->cone_specs,
                                 &c->sweep_blocks, &c->sweep_line, &c->box};
     for (int i = 0; i < kNumBufs; ++i) out[i] = bufs[i];
@@ -1523,14 +1523,10 @@ int solar_gpu_voxelize(solar_gpu_context* c, const float* grid, int W, int H, fl
     CK(cudaSetDevice(c->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : c->own;
     const int T = W * H;
-    RK(ensure(c, c->vox_cnt, sizeof(int) * (size_t)T));
-    RK(ensure(c, c->vox_off, sizeof(long long) * ((size_t)T + 1)));
-    RK(ensure(c, c->vox_tmp, sizeof(long long) * scan_scratch_elems(T)));
-    CK(launch_vox_count(grid, W, H, voxel_size, as<int>(c->vox_cnt), st));
-    CK(launch_scan_counts(as<int>(c->vox_cnt), T, 0, as<long long>(c->vox_off), as<long long>(c->vox_tmp), nullptr,
-                          st));
+    RK(ensure(c, c->vox_off, sizeof(long long) * ((size_t)vox_runs(T) + 1)));
+    CK(launch_vox_count(grid, W, H, voxel_size, as<long long>(c->vox_off), st));
     long long walls = 0;
-    RK(read_ll(c, as<long long>(c->vox_off) + T, &walls, st));
+    RK(read_ll(c, as<long long>(c->vox_off) + vox_runs(T), &walls, st));
     *num_total = (long long)T + walls;
     if (!pixel_parent && !slopes && !aspects) return SOLAR_GPU_OK;   // sizes only
     if (!pixel_parent || !slopes || !aspects || (walls > 0 && !wall_z))

@@ -126,6 +126,8 @@ cudaError_t launch_chunk_order(const int* order, int N, int v0, int n, int* flag
                                long long* scan_tmp, int* perm, cudaStream_t st);
 cudaError_t launch_scan_counts(const int* counts, int n, long long base, long long* offsets,
                                long long* block_sums, int* block_tmp, cudaStream_t st);
+// sums [n + 1]: exclusive scan in place, the total last.
+cudaError_t launch_scan_sums(long long* sums, int n, cudaStream_t st);
 size_t scan_scratch_elems(int n);
 cudaError_t launch_gather_csr(int chunk_count, int D, const int* raw, const long long* offsets,
                               int* csr_ids, const int* inv, cudaStream_t st);
@@ -309,9 +311,10 @@ cudaError_t launch_reflect_mma(const void* slab16, int T, const MmaLists& ml, in
 cudaError_t launch_mma_accumulate(const int* order, int nb, const float* sums, const MmaLists& ml, const Accum& acc,
                                   bool first, bool last, float* out, cudaStream_t st);
 
-// voxelization (voxel.cu): wall voxels per cell, then the packed arrays
-// (tops [0, T), walls after them at T + off[cell] + v).
-cudaError_t launch_vox_count(const float* grid, int W, int H, float voxel_size, int* counts, cudaStream_t st);
+// voxelization (voxel.cu): off [vox_runs(T) + 1], the wall voxels before each run of
+// cells and all of them, then the packed arrays (tops [0, T), walls after them).
+int vox_runs(int T);
+cudaError_t launch_vox_count(const float* grid, int W, int H, float voxel_size, long long* off, cudaStream_t st);
 cudaError_t launch_vox_write(const float* grid, int W, int H, float voxel_size, float scale, const long long* off,
                              int* parent, float* wall_z, float* slopes, float* aspects, cudaStream_t st);
 

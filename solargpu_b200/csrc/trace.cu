@@ -400,6 +400,12 @@ cudaError_t launch_scan_counts(const int* counts, int n, long long base, long lo
     return cudaGetLastError();
 }
 
+cudaError_t launch_scan_sums(long long* sums, int n, cudaStream_t st)
+{
+    k_scan_tile_sums<<<1, kScanThreads, 0, st>>>(sums, n, 0, sums, n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_gather_csr(int chunk_count, int D, const int* raw, const long long* offsets,
                               int* csr_ids, const int* inv, cudaStream_t st)
 {
