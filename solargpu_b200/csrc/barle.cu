@@ -29,8 +29,11 @@
 //
 // Bound: instructions (the sort's shuffles first); the one-lane loops and the
 // run-by-run writes of the two passes were latency.  Sizes, offsets and streams:
-// 160^2 town (35,840 voxels) 0.86 -> 0.28 ms, 512^2 city 9.2 -> 3.0.
+// 160^2 town (35,840 voxels) 0.86 -> 0.24 ms, 512^2 city 9.2 -> 2.0 (3.0 with every
+// loop unrolled, see sort_desc, and a warp a row looking for long lists).
 #include "sgb_internal.cuh"
+
+#include <algorithm>
 
 namespace sgb {
 namespace {
@@ -181,46 +184,52 @@ template <int E>
 __device__ __forceinline__ void sort_desc(uint32_t (&x)[E], int lane)
 {
 #pragma unroll
-    for (int size = 2; size <= 32 * E; size <<= 1) {
-        if (size <= E) {
+    for (int size = 2; size <= E; size <<= 1) {
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            const int m = (j & ~(size - 1)) + size - 1 - (j & (size - 1));
+            if (j < m) swap_desc(x[j], x[m]);
+        }
+#pragma unroll
+        for (int stride = size >> 2; stride > 0; stride >>= 1)
+#pragma unroll
+            for (int j = 0; j < E; ++j)
+                if ((j & stride) == 0) swap_desc(x[j], x[j + stride]);
+    }
+    // The merges over lanes are not unrolled: with all of them in line the kernels
+    // waited on instructions most of the time.
+#pragma unroll 1
+    for (int lanes = 2; lanes <= 32; lanes <<= 1) {
+        const bool above = (lane & (lanes >> 1)) != 0;
+#pragma unroll
+        for (int j = 0; j < E / 2; ++j) {
+            const uint32_t a = __shfl_xor_sync(kAll, x[E - 1 - j], lanes - 1);
+            const uint32_t b = __shfl_xor_sync(kAll, x[j], lanes - 1);
+            x[j] = above ? min(x[j], a) : max(x[j], a);
+            x[E - 1 - j] = above ? min(x[E - 1 - j], b) : max(x[E - 1 - j], b);
+        }
+#pragma unroll 1
+        for (int apart = lanes >> 2; apart > 0; apart >>= 1) {
+            const bool upper = (lane & apart) != 0;
 #pragma unroll
             for (int j = 0; j < E; ++j) {
-                const int m = (j & ~(size - 1)) + size - 1 - (j & (size - 1));
-                if (j < m) swap_desc(x[j], x[m]);
-            }
-        } else {
-            const int lanes = size / E;
-            const bool upper = (lane & (lanes >> 1)) != 0;
-#pragma unroll
-            for (int j = 0; j < E / 2; ++j) {
-                const uint32_t a = __shfl_xor_sync(kAll, x[E - 1 - j], lanes - 1);
-                const uint32_t b = __shfl_xor_sync(kAll, x[j], lanes - 1);
+                const uint32_t a = __shfl_xor_sync(kAll, x[j], apart);
                 x[j] = upper ? min(x[j], a) : max(x[j], a);
-                x[E - 1 - j] = upper ? min(x[E - 1 - j], b) : max(x[E - 1 - j], b);
             }
         }
 #pragma unroll
-        for (int stride = size >> 2; stride > 0; stride >>= 1) {
-            if (stride >= E) {
-                const bool upper = (lane & (stride / E)) != 0;
+        for (int stride = E >> 1; stride > 0; stride >>= 1)
 #pragma unroll
-                for (int j = 0; j < E; ++j) {
-                    const uint32_t a = __shfl_xor_sync(kAll, x[j], stride / E);
-                    x[j] = upper ? min(x[j], a) : max(x[j], a);
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < E; ++j)
-                    if ((j & stride) == 0) swap_desc(x[j], x[j + stride]);
-            }
-        }
+            for (int j = 0; j < E; ++j)
+                if ((j & stride) == 0) swap_desc(x[j], x[j + stride]);
     }
 }
 
-// Encodes k ids (sorted, as sort_desc leaves them) into st; pieces: k words.
-// Returns the stream's bytes.
+// Encodes k ids (sorted, as sort_desc leaves them) into st; pieces: k words,
+// deltas: 32 (E + 1).  Returns the stream's bytes.
 template <int E>
-__device__ __forceinline__ int encode_sorted(uint32_t (&x)[E], int k, unsigned char* st, uint32_t* pieces, int lane)
+__device__ __forceinline__ int encode_sorted(uint32_t (&x)[E], int k, unsigned char* st, uint32_t* pieces,
+                                             uint32_t* deltas, int lane)
 {
     constexpr int kNone = 15;   // class past the list's end
     const int base = lane * E, n = min(max(k - base, 0), E);   // this lane's ids
@@ -288,26 +297,35 @@ __device__ __forceinline__ int encode_sorted(uint32_t (&x)[E], int k, unsigned c
     const uint32_t xr = __shfl_down_sync(kAll, x[0], 1);
     const int apart = __shfl_down_sync(kAll, (n == 0 || (first & 1u)) ? 1 : 0, 1);
     const bool ends = lane == 31 || apart != 0;   // the next lane's first id is in another piece, or past the end
+    // the writes, a loop (see sort_desc): deltas in shared memory, classes 4 bits each
+    unsigned long long wp[(E + 15) / 16];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-        if (j >= n) break;
+        deltas[32 * j + lane] = x[j];
+        if (j % 16 == 0) wp[j / 16] = 0ull;
+        wp[j / 16] |= (unsigned long long)w[j] << (4 * (j % 16));
+    }
+    deltas[32 * E + lane] = xr;   // a lane reads only what it wrote
+#pragma unroll 1
+    for (int j = 0; j < n; ++j) {
+        const int wj = (int)((E > 16 && j >= 16 ? wp[(E - 1) / 16] : wp[0]) >> (4 * (j & 15))) & 15;
+        const uint32_t xj = deltas[32 * j + lane];
         if ((first >> j) & 1u) {
             ++p;
-            pieces[p] = ((uint32_t)b << 14) | (uint32_t)((base + j) << 3) | (uint32_t)w[j];
+            pieces[p] = ((uint32_t)b << 14) | (uint32_t)((base + j) << 3) | (uint32_t)wj;
         }
         // blocks of 8 pieces: 3 bytes of codes and the lengths come before a piece's payload
         const int q = (p >> 3) + 1;
         unsigned char* d = st + b + 3 * q + min(np, 8 * q);
-        if (w[j] == kW4) {
+        if (wj == kW4) {
             if (((odd >> j) & 1u) == 0) {
                 const bool alone = j + 1 < E ? (j + 1 >= n || ((first >> (j + 1)) & 1u)) : ends;
-                const uint32_t y = j + 1 < E ? x[j + 1] : xr;
-                *d = (unsigned char)((x[j] << 4) | (alone ? 0u : y & 0x0Fu));
+                *d = (unsigned char)((xj << 4) | (alone ? 0u : deltas[32 * (j + 1) + lane] & 0x0Fu));
                 ++b;
             }
         } else {
-            for (int i = 0; i < w[j]; ++i) d[i] = (unsigned char)(x[j] >> (8 * (w[j] - 1 - i)));
-            b += w[j];
+            for (int i = 0; i < wj; ++i) d[i] = (unsigned char)(xj >> (8 * (wj - 1 - i)));
+            b += wj;
         }
     }
     __syncwarp();
@@ -329,7 +347,7 @@ __device__ __forceinline__ int encode_sorted(uint32_t (&x)[E], int k, unsigned c
 
 // The list of a row, a lane's ids side by side: sorted, written back, encoded.
 template <int E>
-__device__ __forceinline__ int encode_row(int* row, int k, unsigned char* st, uint32_t* pieces, int lane)
+__device__ __forceinline__ int encode_row(int* row, int k, unsigned char* st, uint32_t* pieces, uint32_t* deltas, int lane)
 {
     uint32_t x[E];
 #pragma unroll
@@ -340,42 +358,87 @@ __device__ __forceinline__ int encode_row(int* row, int k, unsigned char* st, ui
         const int i = lane * E + 4 * j;
         if (i < k) *reinterpret_cast<uint4*>(row + i) = make_uint4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
     }
-    return encode_sorted<E>(x, k, st, pieces, lane);
+    return encode_sorted<E>(x, k, st, pieces, deltas, lane);
 }
 
-// Lists of (E == 16) up to 512, (E == 32) 513 to 1024 ids: size of the stream,
-// which is left in the row after the sorted list.
+// A warp's rows whose lists have more than lo ids: f(row, voxel, ids) for each.  It
+// looks 32 rows over at a time, a count a lane, as far apart as there are warps
+// (long lists are neighbours; side by side, one warp had them all: 160^2 lists 0.56 ms).
+template <typename F>
+__device__ __forceinline__ void for_long_rows(int chunk_count, const int* __restrict__ counts,
+                                              const int* __restrict__ map, int warps, int lane, int lo, F&& f)
+{
+    const int w = blockIdx.x * warps + (threadIdx.x >> 5), apart = gridDim.x * warps;
+    for (long long base = w; base < chunk_count; base += 32LL * apart) {
+        const long long r = base + (long long)lane * apart;
+        const int u = r < chunk_count ? (map ? __ldg(map + r) : (int)r) : 0;
+        const int k = r < chunk_count ? __ldg(counts + u) : 0;
+        unsigned left = __ballot_sync(kAll, k > lo);
+        for (; left; left &= left - 1u) {
+            const int i = __ffs(left) - 1;
+            f((int)base + i * apart, __shfl_sync(kAll, u, i), __shfl_sync(kAll, k, i));
+            __syncwarp();
+        }
+    }
+}
+
+// The stream of a row's list, of up to 32 E ids: its size, and the stream itself in the row
+// after the sorted list.
+template <int E, bool HALF>
+__device__ __forceinline__ void encode_list(int* row, int k, int* size, unsigned char* st, uint32_t* pieces,
+                                            uint32_t* deltas, int lane)
+{
+    const int bytes = HALF && k <= 16 * E ? encode_row<E / 2>(row, k, st, pieces, deltas, lane)
+                                          : encode_row<E>(row, k, st, pieces, deltas, lane);
+    if (lane == 0) *size = bytes;
+    uint4* dst = reinterpret_cast<uint4*>(row + stream_at(k));
+    for (int i = lane; i < (bytes + 15) / 16; i += 32) dst[i] = reinterpret_cast<const uint4*>(st)[i];
+}
+
 template <int E, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32)
+struct EncodeRoom {
+    uint4 st[WARPS][stream_room(32 * E) / 16];
+    uint32_t pieces[WARPS][32 * E], deltas[WARPS][32 * (E + 1)];
+};
+constexpr int kEncodeWarps = 8, kMidWarps = 4;
+
+// Lists of up to 512 ids, a warp a row.
+__global__ void __launch_bounds__(kEncodeWarps * 32)
 k_barle_encode(int chunk_count, int D, int* __restrict__ raw, const int* __restrict__ counts, int* __restrict__ sizes,
                int* __restrict__ err, const int* __restrict__ perm)
 {
-    __shared__ __align__(16) unsigned char s_stream[WARPS][stream_room(32 * E)];
-    __shared__ uint32_t s_pieces[WARPS][32 * E];
+    extern __shared__ __align__(16) unsigned char s_enc[];
+    auto& room = *reinterpret_cast<EncodeRoom<16, kEncodeWarps>*>(s_enc);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int lv = blockIdx.x * WARPS + warp;   // row
+    const int lv = blockIdx.x * kEncodeWarps + warp;   // row
     if (lv >= chunk_count) return;
-    const int u = perm ? perm[lv] : lv;         // voxel of the row
+    const int u = perm ? perm[lv] : lv;                // voxel of the row
     const int k = counts[u];
-    if (E == 32 ? k <= 512 || k > 1024 : k > 512) return;
-    if (E == 16 && k <= 0) {
-        if (lane == 0) sizes[u] = 0;
-        return;
-    }
-    if (k > D) {
+    if (k > 512) return;
+    if (k <= 0 || k > D) {
         if (lane == 0) {
             sizes[u] = 0;
-            atomicOr(err, kErrListCapacity);
+            if (k > D) atomicOr(err, kErrListCapacity);
         }
         return;
     }
-    int* row = raw + (size_t)lv * D;
-    unsigned char* st = s_stream[warp];
-    const int size = E == 16 && k <= 256 ? encode_row<8>(row, k, st, s_pieces[warp], lane)
-                                         : encode_row<E>(row, k, st, s_pieces[warp], lane);
-    if (lane == 0) sizes[u] = size;
-    uint4* dst = reinterpret_cast<uint4*>(row + stream_at(k));
-    for (int i = lane; i < (size + 15) / 16; i += 32) dst[i] = reinterpret_cast<const uint4*>(st)[i];
+    encode_list<16, true>(raw + (size_t)lv * D, k, sizes + u, reinterpret_cast<unsigned char*>(room.st[warp]),
+                          room.pieces[warp], room.deltas[warp], lane);
+}
+
+// Lists of 513 to 1024 ids (D is more, see launch_barle_size).
+__global__ void __launch_bounds__(kMidWarps * 32)
+k_barle_encode_mid(int chunk_count, int D, int* raw, const int* __restrict__ counts, int* sizes,
+                   const int* __restrict__ perm)
+{
+    extern __shared__ __align__(16) unsigned char s_enc[];
+    auto& room = *reinterpret_cast<EncodeRoom<32, kMidWarps>*>(s_enc);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for_long_rows(chunk_count, counts, perm, kMidWarps, lane, 512, [&](int lv, int u, int k) {
+        if (k > kSmallIds) return;
+        encode_list<32, false>(raw + (size_t)lv * D, k, sizes + u, reinterpret_cast<unsigned char*>(room.st[warp]),
+                               room.pieces[warp], room.deltas[warp], lane);
+    });
 }
 
 // The streams of k_barle_encode to their places: whole words there, from pairs
@@ -414,37 +477,34 @@ k_barle_size(int chunk_count, int D, int* __restrict__ raw, const int* __restric
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* ids = smem + warp * (kIdsCap + kRunsCap);
     uint32_t* runs = ids + kIdsCap;
-    const int lv = blockIdx.x * kEncWarps + warp;   // row
-    if (lv >= chunk_count) return;
-    const int u = perm ? perm[lv] : lv;          // voxel of the row
-    const int k = counts[u];
-    if (k <= kSmallIds) return;
-    if (k > D || k > kRunsCap) { if (lane == 0) { sizes[u] = 0; atomicOr(err, kErrListCapacity); } return; }
-    int* row = raw + (size_t)lv * D;
-    load_sorted(row, k, ids, lane, true);
-    for (int i = lane; i < k; i += 32) row[i] = (int)ids[i];   // keep the sorted list for the write pass
-    const int nr = build_runs(ids, k, runs, lane);
-    // and, where the row has room after the list, its optimised runs (the
-    // write pass then skips build_runs): row[k] = run count, runs after it
-    if (k < D) {
-        const bool fits = k + 1 + nr <= D;
-        if (lane == 0) row[k] = fits ? nr : -1;
-        if (fits)
-            for (int r = lane; r < nr; r += 32) row[k + 1 + r] = (int)runs[r];
-    }
-    int pieces = 0, payload = 0;
-    for (int r = lane; r < nr; r += 32) {
-        const int w = run_w(runs[r]), len = run_len(runs[r]);
-        const int full = len / 255, rem = len % 255;
-        pieces += full + (rem > 0);
-        payload += full * payload_bytes(w, 255) + payload_bytes(w, rem);
-    }
+    for_long_rows(chunk_count, counts, perm, kEncWarps, lane, kSmallIds, [&](int lv, int u, int k) {
+        if (k > D || k > kRunsCap) { if (lane == 0) { sizes[u] = 0; atomicOr(err, kErrListCapacity); } return; }
+        int* row = raw + (size_t)lv * D;
+        load_sorted(row, k, ids, lane, true);
+        for (int i = lane; i < k; i += 32) row[i] = (int)ids[i];   // keep the sorted list for the write pass
+        const int nr = build_runs(ids, k, runs, lane);
+        // and, where the row has room after the list, its optimised runs (the
+        // write pass then skips build_runs): row[k] = run count, runs after it
+        if (k < D) {
+            const bool fits = k + 1 + nr <= D;
+            if (lane == 0) row[k] = fits ? nr : -1;
+            if (fits)
+                for (int r = lane; r < nr; r += 32) row[k + 1 + r] = (int)runs[r];
+        }
+        int pieces = 0, payload = 0;
+        for (int r = lane; r < nr; r += 32) {
+            const int w = run_w(runs[r]), len = run_len(runs[r]);
+            const int full = len / 255, rem = len % 255;
+            pieces += full + (rem > 0);
+            payload += full * payload_bytes(w, 255) + payload_bytes(w, rem);
+        }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        pieces += __shfl_xor_sync(0xFFFFFFFFu, pieces, o);
-        payload += __shfl_xor_sync(0xFFFFFFFFu, payload, o);
-    }
-    if (lane == 0) sizes[u] = 3 * ((pieces + 7) / 8) + pieces + payload;
+        for (int o = 16; o > 0; o >>= 1) {
+            pieces += __shfl_xor_sync(0xFFFFFFFFu, pieces, o);
+            payload += __shfl_xor_sync(0xFFFFFFFFu, payload, o);
+        }
+        if (lane == 0) sizes[u] = 3 * ((pieces + 7) / 8) + pieces + payload;
+    });
 }
 
 __global__ void __launch_bounds__(kEncWarps * 32)
@@ -456,84 +516,90 @@ k_barle_write(int chunk_count, int D, const int* __restrict__ raw, const int* __
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* ids = smem + warp * (kIdsCap + kRunsCap);
     uint32_t* runs = ids + kIdsCap;
-    const int lv = blockIdx.x * kEncWarps + warp;
-    if (lv >= chunk_count) return;
-    const int k = counts[lv];
-    if (k <= kSmallIds) return;
-    if (k > D || k > kRunsCap) return;
-    const int* row = raw + (size_t)(inv ? inv[lv] : lv) * D;
-    load_sorted(row, k, ids, lane, false);   // already sorted by k_barle_size
-    // the runs k_barle_size left after the list, else built again
-    int nr = k < D ? row[k] : -1;
-    if (nr >= 0 && k + 1 + nr <= D) {
-        for (int r = lane; r < nr; r += 32) runs[r] = (uint32_t)row[k + 1 + r];
-        __syncwarp();
-    } else {
-        nr = build_runs(ids, k, runs, lane);
-    }
-    // split_long_runs (barle_compression.cpp:29-44), expanded in place from the back
-    if (lane == 0) {
-        int ns = 0;
-        for (int r = 0; r < nr; ++r) ns += (run_len(runs[r]) + 254) / 255;
-        int pos = ns;
-        for (int r = nr - 1; r >= 0; --r) {
-            const int w = run_w(runs[r]), len = run_len(runs[r]);
-            const int np = (len + 254) / 255;
-            pos -= np;
-            for (int p = np - 1; p >= 0; --p) {
-                const int pl = (p == np - 1) ? len - 255 * (np - 1) : 255;
-                runs[pos + p] = pack_run(w, pl);
-            }
-        }
-        nr = ns;
-    }
-    nr = __shfl_sync(0xFFFFFFFFu, nr, 0);
-    __syncwarp();
-    unsigned char* dst = out + offsets[lv];
-    const long long limit = offsets[lv + 1] - offsets[lv];
-    long long boff = 0;
-    int estart = 0;
-    for (int p = 0; p < nr; ++p) {
-        if ((p & 7) == 0) {
-            const int cnt = min(8, nr - p);
-            if (lane == 0) {
-                uint32_t bits = 0;
-                for (int j = 0; j < 8; ++j) {
-                    const int code = (j < cnt) ? run_w(runs[p + j]) : kEnd;
-                    bits |= (uint32_t)(code & 7) << ((7 - j) * 3);
-                }
-                if (boff + 3 + cnt <= limit) {
-                    dst[boff] = (unsigned char)(bits >> 16);
-                    dst[boff + 1] = (unsigned char)(bits >> 8);
-                    dst[boff + 2] = (unsigned char)bits;
-                }
-            }
-            if (lane < cnt && boff + 3 + cnt <= limit) dst[boff + 3 + lane] = (unsigned char)run_len(runs[p + lane]);
-            boff += 3 + cnt;
-        }
-        const int w = run_w(runs[p]), len = run_len(runs[p]);
-        const int nb = payload_bytes(w, len);
-        if (boff + nb > limit) { if (lane == 0) atomicOr(err, kErrListCapacity); return; }
-        if (w == kW4) {
-            for (int b = lane; b < nb; b += 32) {
-                const int e = estart + 2 * b;
-                const uint32_t v1 = delta_at(ids, e);
-                const uint32_t v2 = (2 * b + 1 < len) ? delta_at(ids, e + 1) : 0u;
-                dst[boff + b] = (unsigned char)((v1 << 4) | (v2 & 0x0Fu));
-            }
+    for_long_rows(chunk_count, counts, nullptr, kEncWarps, lane, kSmallIds, [&](int lv, int, int k) {
+        if (k > D || k > kRunsCap) return;
+        const int* row = raw + (size_t)(inv ? inv[lv] : lv) * D;
+        load_sorted(row, k, ids, lane, false);   // already sorted by k_barle_size
+        // the runs k_barle_size left after the list, else built again
+        int nr = k < D ? row[k] : -1;
+        if (nr >= 0 && k + 1 + nr <= D) {
+            for (int r = lane; r < nr; r += 32) runs[r] = (uint32_t)row[k + 1 + r];
+            __syncwarp();
         } else {
-            for (int i = lane; i < len; i += 32) {
-                const uint32_t x = delta_at(ids, estart + i);
-                unsigned char* q = dst + boff + (long long)i * w;
-                for (int b = 0; b < w; ++b) q[b] = (unsigned char)(x >> (8 * (w - 1 - b)));
-            }
+            nr = build_runs(ids, k, runs, lane);
         }
-        boff += nb;
-        estart += len;
-    }
+        // split_long_runs (barle_compression.cpp:29-44), expanded in place from the back
+        if (lane == 0) {
+            int ns = 0;
+            for (int r = 0; r < nr; ++r) ns += (run_len(runs[r]) + 254) / 255;
+            int pos = ns;
+            for (int r = nr - 1; r >= 0; --r) {
+                const int w = run_w(runs[r]), len = run_len(runs[r]);
+                const int np = (len + 254) / 255;
+                pos -= np;
+                for (int p = np - 1; p >= 0; --p) {
+                    const int pl = (p == np - 1) ? len - 255 * (np - 1) : 255;
+                    runs[pos + p] = pack_run(w, pl);
+                }
+            }
+            nr = ns;
+        }
+        nr = __shfl_sync(0xFFFFFFFFu, nr, 0);
+        __syncwarp();
+        unsigned char* dst = out + offsets[lv];
+        const long long limit = offsets[lv + 1] - offsets[lv];
+        long long boff = 0;
+        int estart = 0;
+        for (int p = 0; p < nr; ++p) {
+            if ((p & 7) == 0) {
+                const int cnt = min(8, nr - p);
+                if (lane == 0) {
+                    uint32_t bits = 0;
+                    for (int j = 0; j < 8; ++j) {
+                        const int code = (j < cnt) ? run_w(runs[p + j]) : kEnd;
+                        bits |= (uint32_t)(code & 7) << ((7 - j) * 3);
+                    }
+                    if (boff + 3 + cnt <= limit) {
+                        dst[boff] = (unsigned char)(bits >> 16);
+                        dst[boff + 1] = (unsigned char)(bits >> 8);
+                        dst[boff + 2] = (unsigned char)bits;
+                    }
+                }
+                if (lane < cnt && boff + 3 + cnt <= limit) dst[boff + 3 + lane] = (unsigned char)run_len(runs[p + lane]);
+                boff += 3 + cnt;
+            }
+            const int w = run_w(runs[p]), len = run_len(runs[p]);
+            const int nb = payload_bytes(w, len);
+            if (boff + nb > limit) { if (lane == 0) atomicOr(err, kErrListCapacity); return; }
+            if (w == kW4) {
+                for (int b = lane; b < nb; b += 32) {
+                    const int e = estart + 2 * b;
+                    const uint32_t v1 = delta_at(ids, e);
+                    const uint32_t v2 = (2 * b + 1 < len) ? delta_at(ids, e + 1) : 0u;
+                    dst[boff + b] = (unsigned char)((v1 << 4) | (v2 & 0x0Fu));
+                }
+            } else {
+                for (int i = lane; i < len; i += 32) {
+                    const uint32_t x = delta_at(ids, estart + i);
+                    unsigned char* q = dst + boff + (long long)i * w;
+                    for (int b = 0; b < w; ++b) q[b] = (unsigned char)(x >> (8 * (w - 1 - b)));
+                }
+            }
+            boff += nb;
+            estart += len;
+        }
+    });
 }
 
 }  // namespace
+
+// Blocks (of 4 warps) of the kernels for long lists: a warp for 32 rows, and small
+// scenes fill the GPU.  A warp a row took 0.45 ms at 512^2 to find none above 1024.
+static int long_blocks(int rows)
+{
+    static_assert(kEncWarps == 4 && kMidWarps == 4, "blocks of 4 warps");
+    return std::max(std::min((rows + 3) / 4, 3 * 148), (rows + 127) / 128);
+}
 
 cudaError_t launch_barle_size(int chunk_count, int D, int* raw, const int* counts, int* sizes, int* err,
                               const int* perm, cudaStream_t st)
@@ -541,15 +607,18 @@ cudaError_t launch_barle_size(int chunk_count, int D, int* raw, const int* count
     if (chunk_count <= 0) return cudaSuccess;
     // a row holds the list and the stream of up to kSmallIds ids, and starts on 16 bytes
     if (D % 4 != 0 || 4 * D < 4 * kSmallIds + stream_room(kSmallIds)) return cudaErrorInvalidValue;
-    k_barle_encode<16, 8><<<(chunk_count + 7) / 8, 8 * 32, 0, st>>>(chunk_count, D, raw, counts, sizes, err, perm);
-    k_barle_encode<32, 4><<<(chunk_count + 3) / 4, 4 * 32, 0, st>>>(chunk_count, D, raw, counts, sizes, err, perm);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    constexpr size_t room = sizeof(EncodeRoom<16, kEncodeWarps>), mid = sizeof(EncodeRoom<32, kMidWarps>);
     constexpr size_t smem = (size_t)kEncWarps * (kIdsCap + kRunsCap) * sizeof(uint32_t);
-    e = cudaFuncSetAttribute(k_barle_size, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_barle_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_barle_encode_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mid);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_barle_size, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_barle_size<<<(chunk_count + kEncWarps - 1) / kEncWarps, kEncWarps * 32, smem, st>>>(chunk_count, D, raw, counts,
-                                                                                         sizes, err, perm);
+    k_barle_encode<<<(chunk_count + kEncodeWarps - 1) / kEncodeWarps, kEncodeWarps * 32, room, st>>>(
+        chunk_count, D, raw, counts, sizes, err, perm);
+    k_barle_encode_mid<<<long_blocks(chunk_count), kMidWarps * 32, mid, st>>>(
+        chunk_count, D, raw, counts, sizes, perm);
+    k_barle_size<<<long_blocks(chunk_count), kEncWarps * 32, smem, st>>>(chunk_count, D, raw, counts, sizes, err, perm);
     return cudaGetLastError();
 }
 
@@ -565,7 +634,7 @@ cudaError_t launch_barle_write(int chunk_count, int D, const int* raw, const int
     constexpr size_t smem = (size_t)kEncWarps * (kIdsCap + kRunsCap) * sizeof(uint32_t);
     e = cudaFuncSetAttribute(k_barle_write, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_barle_write<<<(chunk_count + kEncWarps - 1) / kEncWarps, kEncWarps * 32, smem, st>>>(
+    k_barle_write<<<long_blocks(chunk_count), kEncWarps * 32, smem, st>>>(
         chunk_count, D, raw, counts, offsets, out, err, inv);
     return cudaGetLastError();
 }
