@@ -796,10 +796,14 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
             RK(ensure(c, c->w_cnt, sizeof(int) * (size_t)N));
             RK(ensure(c, c->w_off, sizeof(long long) * ((size_t)N + 1)));
             RK(ensure(c, c->w_tmp, sizeof(long long) * scan_scratch_elems(N)));
+            // the raw hit rows are dead by now, if there are any (saved lists come without)
+            ListRoom room{nullptr, (int)sky.dirs.size() / 2};
+            if (nl.format == SOLAR_GPU_BARLE && c->raw.cap >= sizeof(int2) * (size_t)N * room.per)
+                room.rows = as<int2>(c->raw);
             {
                 KScope k(c, SOLAR_GPU_KT_GROUP);
                 CK(launch_weight_lists(0, g, N, T, nl, as<int>(c->order), as<int>(c->w_cnt), nullptr, nullptr,
-                                       nullptr, err, st));
+                                       nullptr, room, err, st));
                 CK(launch_scan_counts(as<int>(c->w_cnt), N, 0, as<long long>(c->w_off), as<long long>(c->w_tmp),
                                       nullptr, st));
             }
@@ -811,7 +815,7 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
             {
                 KScope k(c, SOLAR_GPU_KT_GROUP);
                 CK(launch_weight_lists(1, g, N, T, nl, as<int>(c->order), nullptr, as<long long>(c->w_off),
-                                       as<int>(c->w_cell), as<float>(c->w_val), err, st));
+                                       as<int>(c->w_cell), as<float>(c->w_val), room, err, st));
             }
             c->launches += 5;
             if (mma) {
@@ -859,7 +863,7 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
                     V = 64;
                     KScope k(c, SOLAR_GPU_KT_GROUP);
                     CK(launch_weight_lists(1, g, N, T, nl, as<int>(c->order), nullptr, as<long long>(c->w_off),
-                                           as<int>(c->w_cell), as<float>(c->w_val), err, st));
+                                           as<int>(c->w_cell), as<float>(c->w_val), room, err, st));
                     c->launches += 1;
                 } else {
                     RK(ensure(c, c->mma_ccnt, sizeof(int) * (size_t)(C + 1)));

@@ -199,10 +199,15 @@ struct GroupLists {
 };
 int group_count(int N, int V);
 // Weighted lists in visiting order: pass 0 counts nonzero weights per
-// position, pass 1 writes (cell, w) at woff[p].
+// position, pass 1 writes (cell, w) at woff[p].  room: rows for pass 0 to keep the
+// first `per` of a position's (cell, w) for pass 1, or none (rows == nullptr).
+struct ListRoom {
+    int2* rows;
+    int per;
+};
 cudaError_t launch_weight_lists(int pass, const DevGeom& g, int N, int T, const NeighborLists& nl,
                                 const int* order, int* counts, const long long* woff, int* cells,
-                                float* wts, int* err, cudaStream_t st);
+                                float* wts, const ListRoom& room, int* err, cudaStream_t st);
 // Merges the weighted lists of V consecutive positions into union entries.
 cudaError_t launch_group_merge(int pass, int V, int N, const long long* woff, const int* wcell,
                                const float* wts, int* counts, const long long* goff, int* cell, float* w,
