@@ -335,6 +335,32 @@ k_gather_csr(int chunk_count, int D, const int* __restrict__ raw, const long lon
     for (int i = lane; i < k; i += 32) csr_ids[o + i] = row[i];
 }
 
+// Scans of up to kScanOne counts in one block: one launch for three (64^2 runs have
+// five such scans: 884 -> 860 us).
+constexpr int kScanOne = 16 * kScanThreads;
+
+__global__ void __launch_bounds__(kScanThreads)
+k_scan_one(const int* __restrict__ counts, int n, long long base, long long* __restrict__ offsets)
+{
+    constexpr int kItems = kScanOne / kScanThreads;
+    const int per = (n + kScanThreads - 1) / kScanThreads, at = threadIdx.x * per;
+    int v[kItems];
+    long long local = 0;
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+        v[i] = i < per && at + i < n ? counts[at + i] : 0;
+        local += v[i];
+    }
+    long long total;
+    long long run = base + block_excl_scan(local, &total);
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+        if (i < per && at + i < n) offsets[at + i] = run;
+        run += v[i];
+    }
+    if (threadIdx.x == 0) offsets[n] = base + total;
+}
+
 }  // namespace
 
 cudaError_t launch_pad_grid(const float* grid, int W, int H, float* gpad, cudaStream_t st)
@@ -393,6 +419,10 @@ size_t scan_scratch_elems(int n)
 cudaError_t launch_scan_counts(const int* counts, int n, long long base, long long* offsets,
                                long long* block_sums, int* /*unused*/, cudaStream_t st)
 {
+    if (n > 0 && n <= kScanOne) {
+        k_scan_one<<<1, kScanThreads, 0, st>>>(counts, n, base, offsets);
+        return cudaGetLastError();
+    }
     const int ntiles = (n + kScanTile - 1) / kScanTile;
     if (n > 0) k_scan_tiles<<<ntiles, kScanThreads, 0, st>>>(counts, n, offsets, block_sums);
     k_scan_tile_sums<<<1, kScanThreads, 0, st>>>(block_sums, ntiles, base, offsets, n);
