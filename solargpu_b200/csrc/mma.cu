@@ -55,11 +55,13 @@
 // k_mma_accumulate then adds up each voxel's hour blocks (FP64, Kahan or plain).
 //
 // Bound: the MMAs, and FP32 issue in k_light.  A chunk's eight MMAs take 1024 cycles
-// of the tensor pipe (measured alone, B MN-major or K-major alike); here a chunk takes
-// about 1800, where it took 2300 to 2500 with one launch an hour block, one
+// of the tensor pipe (measured alone, B MN-major or K-major alike), reading 96 KB of
+// shared memory that the staging writes as much to; with all cells in the unions
+// a chunk took 1630 to 1800 here, and 2300 to 2500 with one launch an hour block, one
 // builder team, the own terms in the epilogue and each chunk published after the
 // wait for the stage of the chunk two ahead.  Without the light cells a chunk has 2.5
-// times the entries: three builder teams take 21.1 ms at 1024^2 where two took 22.9.
+// times the entries and takes about 2200: three builder teams take 21.1 ms at 1024^2
+// where two took 22.9 (light cells of up to 6 entries).
 // Reflection of the 1024^2 city 78.5 ms at first, 58.6 with all cells in the
 // unions, 30.8 with light cells; 512^2 20.1, 13.0 and 7.3; 160^2 2.38, 1.13 and 0.73.
 //

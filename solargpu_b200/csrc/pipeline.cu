@@ -147,6 +147,9 @@ struct solar_gpu_context {
     // solar_gpu_run_batch: the early-exit tables of every tile are built in
     // one buffer (the first context's), tile after tile on one stream
     DevBuf* cone_shared = nullptr;
+    // and so are the raw hit rows, dead once a tile's lists are built (the rows of 32
+    // tiles at once, 130 GB of them, left no room for the rest)
+    DevBuf* raw_shared = nullptr;
     // origin classes of the tracer's tables in sweep_blocks / sweep_line (0:
     // none built); in a batch, the first context's tables serve every tile
     int sweep_ne = 0;
@@ -188,6 +191,9 @@ int check_limit(solar_gpu_context* c, size_t extra)
                     held, extra);
     return SOLAR_GPU_OK;
 }
+
+// The raw hit rows the context works in.
+DevBuf& raw_rows(solar_gpu_context* c) { return c->raw_shared ? *c->raw_shared : c->raw; }
 
 int ensure(solar_gpu_context* c, DevBuf& b, size_t bytes)
 {
@@ -388,12 +394,13 @@ long long auto_chunk(solar_gpu_context* c, int N, int D)
     // A raw buffer kept from an earlier call that holds the whole scene is
     // reused without asking the driver for free memory (that query can wait
     // behind other processes' driver calls, e.g. monitoring tools).
-    if (c->raw.cap >= sizeof(int) * (size_t)N * D) return N;
+    const DevBuf& raw = raw_rows(c);
+    if (raw.cap >= sizeof(int) * (size_t)N * D) return N;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = (size_t)8 << 30;
     if (c->mem_limit > 0) {
         // under a memory limit: what the limit leaves, counting the raw buffer's current size as free
-        const size_t held = held_bytes(c) - c->raw.cap;
+        const size_t held = held_bytes(c) - raw.cap;
         const size_t room = (size_t)c->mem_limit > held ? (size_t)c->mem_limit - held : 0;
         if (room < free_b) free_b = room;
     }
@@ -427,7 +434,8 @@ int padded_grid(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables&
     DevBuf& tabs = c->cone_shared ? *c->cone_shared : c->cone;
     const size_t bytes = sizeof(float) * cells * (size_t)nt;
     const size_t scratch = sizeof(float) * cone_scratch(W, H, nt);
-    const bool scratch_in_raw = c->raw.cap >= scratch;
+    DevBuf& raw = raw_rows(c);
+    const bool scratch_in_raw = raw.cap >= scratch;
     // device memory these tables would add to what the context holds
     const size_t grow = (bytes > tabs.cap ? bytes - tabs.cap : 0) +
                         (!scratch_in_raw && scratch > c->cone_tmp.cap ? scratch - c->cone_tmp.cap : 0);
@@ -454,7 +462,7 @@ int padded_grid(solar_gpu_context* c, const solar_gpu_scene* s, const SkyTables&
     RK(ensure(c, c->cone_specs, sizeof(ConeSpec) * nt));
     CK(cudaMemcpyAsync(c->cone_specs.p, sky.cones.data(), sizeof(ConeSpec) * nt, cudaMemcpyHostToDevice, st));
     CK(launch_cone_tables(s->grid, W, H, s->max_height, as<ConeSpec>(c->cone_specs), nt, as<float>(tabs),
-                          scratch_in_raw ? as<float>(c->raw) : as<float>(c->cone_tmp), cells, st));
+                          scratch_in_raw ? as<float>(raw) : as<float>(c->cone_tmp), cells, st));
     c->launches += 6;
     ds.cone = as<float>(tabs);
     ds.cone_stride = cells;
@@ -528,7 +536,8 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
     c->csr_total = c->barle_total = 0;
     RK(ensure(c, c->shadow, sizeof(uint32_t) * (size_t)N * c->words32));
     CK(cudaMemsetAsync(c->shadow.p, 0, sizeof(uint32_t) * (size_t)N * c->words32, st));
-    RK(ensure(c, c->raw, sizeof(int) * (size_t)chunk * D));
+    DevBuf& raw = raw_rows(c);
+    RK(ensure(c, raw, sizeof(int) * (size_t)chunk * D));
     RK(ensure(c, c->counts, sizeof(int) * (size_t)N));
     RK(ensure(c, c->dd_ovf, sizeof(int) * ((size_t)chunk + 1)));
     RK(ensure(c, c->scan_tmp, sizeof(long long) * scan_scratch_elems((int)chunk)));
@@ -580,12 +589,12 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
         }
         {
             KScope k(c, SOLAR_GPU_KT_TRACE);
-            CK(trace_rows(sweep, ds, as<DirEntry>(c->dirs), D, c->words32, (int)v0, n, as<int>(c->raw),
+            CK(trace_rows(sweep, ds, as<DirEntry>(c->dirs), D, c->words32, (int)v0, n, as<int>(raw),
                           as<uint32_t>(c->shadow), perm, as<int>(c->err), st));
         }
         {
             KScope k(c, SOLAR_GPU_KT_DEDUPE);
-            CK(launch_dedupe(n, D, as<int>(c->raw), as<int>(c->counts) + v0, as<int>(c->err), perm,
+            CK(launch_dedupe(n, D, as<int>(raw), as<int>(c->counts) + v0, as<int>(c->err), perm,
                              as<int>(c->dd_ovf), st));
         }
         c->launches += 2;
@@ -602,7 +611,7 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
             RK(ensure_keep(c, c->csr_ids, sizeof(int) * (size_t)(est > total ? est : total), sizeof(int) * (size_t)csr_total, st));
             {
                 KScope k(c, SOLAR_GPU_KT_CSR);
-                CK(launch_gather_csr(n, D, as<int>(c->raw), off, as<int>(c->csr_ids), inv, st));
+                CK(launch_gather_csr(n, D, as<int>(raw), off, as<int>(c->csr_ids), inv, st));
             }
             csr_total = total;
             c->launches += 4;
@@ -611,7 +620,7 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
             long long* off = as<long long>(c->barle_off) + v0;
             {
                 KScope k(c, SOLAR_GPU_KT_BARLE);
-                CK(launch_barle_size(n, D, as<int>(c->raw), as<int>(c->counts) + v0, as<int>(c->barle_sizes) + v0,
+                CK(launch_barle_size(n, D, as<int>(raw), as<int>(c->counts) + v0, as<int>(c->barle_sizes) + v0,
                                      as<int>(c->err), perm, st));
                 CK(launch_scan_counts(as<int>(c->barle_sizes) + v0, n, barle_total, off, as<long long>(c->scan_tmp), nullptr, st));
             }
@@ -621,7 +630,7 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
             RK(ensure_keep(c, c->barle_bytes, (size_t)(est > total ? est : total), (size_t)barle_total, st));
             {
                 KScope k(c, SOLAR_GPU_KT_BARLE);
-                CK(launch_barle_write(n, D, as<int>(c->raw), as<int>(c->counts) + v0, off,
+                CK(launch_barle_write(n, D, as<int>(raw), as<int>(c->counts) + v0, off,
                                       as<unsigned char>(c->barle_bytes), as<int>(c->err), inv, st));
             }
             barle_total = total;
@@ -633,10 +642,10 @@ int stage1(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sce
     // A raw hit buffer above a quarter of the device (scenes of tens of
     // millions of voxels) is released here to leave room for Stage 2/3;
     // smaller ones are kept for the next call.
-    if (c->raw.cap > c->dev_total / 4) {
+    if (raw.cap > c->dev_total / 4) {
         c->squeezed = true;
         c->sweep_ne = 0;
-        for (DevBuf* b : {&c->raw, &c->cone, &c->cone_tmp, &c->sweep_blocks, &c->sweep_line, &c->box}) {
+        for (DevBuf* b : {&raw, &c->cone, &c->cone_tmp, &c->sweep_blocks, &c->sweep_line, &c->box}) {
             CK(cudaFree(b->p));
             b->p = nullptr;
             b->cap = 0;
@@ -807,8 +816,8 @@ int stage23(solar_gpu_context* c, const solar_gpu_options* o, const solar_gpu_sc
             RK(ensure(c, c->w_tmp, sizeof(long long) * scan_scratch_elems(N)));
             // the raw hit rows are dead by now, if there are any (saved lists come without)
             ListRoom room{nullptr, (int)sky.dirs.size() / 2};
-            if (nl.format == SOLAR_GPU_BARLE && c->raw.cap >= sizeof(int2) * (size_t)N * room.per)
-                room.rows = as<int2>(c->raw);
+            if (nl.format == SOLAR_GPU_BARLE && raw_rows(c).cap >= sizeof(int2) * (size_t)N * room.per)
+                room.rows = as<int2>(raw_rows(c));
             {
                 KScope k(c, SOLAR_GPU_KT_GROUP);
                 CK(launch_weight_lists(0, g, N, T, nl, as<int>(c->order), as<int>(c->w_cnt), nullptr, nullptr,
@@ -1539,6 +1548,9 @@ int solar_gpu_run_batch(solar_gpu_context* const* ctxs, int n, const solar_gpu_o
             return fail(SOLAR_GPU_ERR_ARG, "a batch runs the hour-block path (hour_block > 1, hourly reflection)");
     CK(cudaSetDevice(ctxs[0]->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : ctxs[0]->own;
+    // a memory limit counts a context's own buffers, so then each has its own rows
+    bool limited = false;
+    for (int i = 0; i < n; ++i) limited = limited || ctxs[i]->mem_limit > 0;
     // Stage 1 and the once-per-run builds, tile after tile (each sizes its
     // buffers from its own lists); each stops before its hour loop.
     for (int i = 0; i < n; ++i) {
@@ -1547,10 +1559,12 @@ int solar_gpu_run_batch(solar_gpu_context* const* ctxs, int n, const solar_gpu_o
         ob.time_kernels = 0;
         c->defer_hours = true;
         c->sweep_owner = ctxs[0];
+        c->raw_shared = limited ? nullptr : &ctxs[0]->raw;   // as the tables:
         c->cone_shared = &ctxs[0]->cone;   // one stream: tile i's tables are built after tile i - 1 is traced
         const int rc = run_device_impl(c, &ob, &scenes[i], outs[i], st, false);
         c->defer_hours = false;
         c->cone_shared = nullptr;
+        c->raw_shared = nullptr;
         c->sweep_owner = nullptr;
         if (rc != SOLAR_GPU_OK) return rc;
     }
